@@ -96,7 +96,7 @@ def draw(rng):
         return {"do": do, "batch": _log(rng, 1, 128), "n_min": _log(rng, 2048, 16384),
                 "step": round(math.exp(rng.uniform(math.log(0.2), math.log(4.0))), 3), "top": rng.randint(10, 200)}
     if do == "plain":
-        n = _log(rng, 1024, 6000)
+        n = _log(rng, 1024, 3001)
         return {"do": do, "batch": _log(rng, 1, 48), "n_min": n, "n_max": n, "n_trial": _log(rng, 128, 4096),
                 "kind": "morse", "psi": rng.random() < 0.5}
     if do == "long":
