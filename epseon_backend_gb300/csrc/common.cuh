@@ -25,6 +25,10 @@
 
 namespace epscu {
 
+// the fast method's level lists (LevelWork::bucket / kBuckets), each ordered by
+// window-length classes (quarter octaves)
+enum { kListWarp = 0, kListLong, kListFragile, kListFragileLong, kLists };
+constexpr int kBuckets = 64;
 constexpr int kRenorm = 32;  // renormalise the projective state every kRenorm steps
 
 // Per-potential constants, written by the prepare kernel.
@@ -57,6 +61,7 @@ struct LevelWork {
     int32_t iters;
     int32_t j0, j1;     // grid window of the level's passes ([i0, i1] unless narrowed
                         // by the decay window of the fast method)
+    int32_t bucket, rank;  // fast method: place in the order of falling window length
     int32_t n_in_bracket;  // levels the scan counted inside the scan bracket
     int32_t pad1;
 };
@@ -73,8 +78,11 @@ struct Header {
     int32_t n_twist;        // levels handed to the twist-index search
     int32_t queue[16];      // work-queue heads of the per-level kernels
     int32_t n_long;         // levels whose window takes the CTA-per-level passes
-    int32_t n_mid;          // levels whose window takes the warp-per-level passes
-    int32_t pad_mid;
+    int32_t n_warp;         // levels whose window takes the warp-per-level passes
+    int32_t n_fragile;       // fragile levels on lanes, those with long windows,
+    int32_t n_fragile_long;
+    int32_t n_fragile_fall;  //   those the lane Newton handed over,
+    int32_t n_fragile_twist; //   those for the twist-index search
     int32_t bis_items_n;    // bisection round: (potential, chunk) items listed
     int32_t bis_items_q;    //   and the work-queue head over them
     int32_t n_redo;         // norm passes redone at E + dE
@@ -86,25 +94,26 @@ struct Header {
     unsigned long long df_max_updates;      // largest per-level point-updates of newton_df / norm_df
     int32_t refine_max_iters;               // most refine32 passes of one level
     int32_t pad_hdr;
-    unsigned long long long32_updates;      // refine_long (long list): FP32 pass point-updates
+    int32_t hist[kLists * kBuckets];        // levels by list and window length
+    unsigned long long long32_updates;      // CTA levels: FP32 pass point-updates
     unsigned long long longdf_updates;      //   and double-float pass point-updates
-    unsigned long long psi_zero_points;     // psi points zeroed by zero_psi (outside the windows)
-    unsigned long long psi_window_points;   // window points scale_psi converted
+    unsigned long long psi_zero_points;     // psi points zeroed (outside the windows)
+    unsigned long long psi_window_points;   // window points written
 };
 
 // queue ids of the per-level kernels
-enum { kQRefine32 = 0, kQNewtonDF, kQNormDF, kQWriteDF, kQBisect64, kQNorm64, kQWrite64, kQLongRefine, kQFallback,
-       kQNormLong, kQTwistLong, kQMidRefine, kQNormMid, kQScalePsi, kQNormFallback };
+enum { kQBisect64 = 0, kQNorm64, kQWrite64, kQWarpLevels, kQLongLevels, kQRepair, kQWarpRewrite, kQLongRewrite,
+       kQFragileLanes, kQFragileLong, kQFragileRepair, kQFragileRewrite };
 
 // internal level flags (not reported: gather keeps the public bits only)
-// the Newton stage handed the level to the fallback: its refinement, norm pass
-// and (recompute) write run one CTA per level over the fallback list, and its
-// norm constants are the group passes' (the lane kernels skip it)
-#define EPSCU_STATUS_FALLBACK 0x10000
-// the level's passes run one CTA per level (longwin.cu)
+// the level's final passes ran one CTA per level
 #define EPSCU_STATUS_LONG 0x20000
-// the level's double-float passes run one warp per level (the middle tier, longwin.cu)
-#define EPSCU_STATUS_MID 0x40000
+// (fragile.cu) the lane Newton handed the level over: its refinement, norm pass
+// and rewrite run on a CTA (the lane passes skip it)
+#define EPSCU_STATUS_FALLBACK 0x10000
+// (potential) a point inside the cut-offs lies above them: 1 + T can be small
+// there, and a fast pass renormalises after every point
+#define EPSCU_STATUS_STEEP 0x40000
 #define EPSCU_STATUS_PUBLIC 0xffff
 // spacing of the samples of the twist-index search
 constexpr int kTwistSample = 64;

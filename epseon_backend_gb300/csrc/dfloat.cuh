@@ -102,7 +102,13 @@ struct SqSum {
     }
     __device__ __forceinline__ void add(dfl v) { d = df_add(d, v); }
     __device__ __forceinline__ void rescale(int s) {
-        if (s == 0) return;
+        if (x == 0.0 && d.h == 0.0f) return;
+        const int ex = fexp(d.h) + s;
+        if (x == 0.0 && s > -120 && s < 120 && ex > -100 && ex < 100) d = df_scale(d, fpow2(s));
+        else rescale_spill(s);
+    }
+    // (a call: rare, and the inlined FP64 path tripled the norm pass's code)
+    __device__ __noinline__ void rescale_spill(int s) {
         if (x != 0.0) {
             pend += s;
             if (pend < -1000) {  // the spilled part fell below any contribution
@@ -165,6 +171,8 @@ __device__ __forceinline__ double df_pair_to_double(float h, float l) {
                                             (M & 0xfffffffffffffull)));
 }
 
+static __device__ __noinline__ double ldexp_call(double d, int e) { return ldexp(d, e); }
+
 // df_pair_to_double(h, l) * 2^e2, the exponent added in the bits while the
 // result stays a normal double (ldexp otherwise)
 __device__ __forceinline__ double df_pair_to_double_scaled(float h, float l, int e2) {
@@ -174,7 +182,7 @@ __device__ __forceinline__ double df_pair_to_double_scaled(float h, float l, int
     if (ex == 0) return d;  // zero (a subnormal pair product: below any psi value)
     const int en = ex + e2;
     if (en >= 1 && en <= 2046) return __longlong_as_double(u + ((long long)e2 << 52));
-    return ldexp(d, e2);
+    return ldexp_call(d, e2);
 }
 
 // A double as a double-float pair (h + l, ~48 significant bits) through its

@@ -1,5 +1,5 @@
-// dfpass.cuh -- pieces shared by the double-float passes of the fast method
-// (polish.cu: one lane per level; longwin.cu: one CTA per long level).
+// dfpass.cuh -- pieces shared by the fast method's per-level passes
+// (levelpass.cu, fragile.cu).
 #pragma once
 
 #include <math.h>
@@ -10,31 +10,14 @@
 
 namespace epscu {
 
-// Windows longer than a threshold take the CTA-per-level passes of
-// longwin.cu (parallel prefix over chunks) instead of one lane per level.  A
-// lane marching a long window is the tail of the per-level kernels: its
-// latency, not the throughput, sets their duration; the CTA passes cost ~3x
-// the point-updates in double-float but cut the latency ~80x.  So the
-// threshold falls with the number of levels (fewer lanes to keep the GPU
-// busy): 8192 points at >= ~9e4 levels (the 2048-potential mixed batch),
-// proportionally less below, never under 1024.  Measured on GB300 with the
-// long levels on their own stream beside the lane kernels and FP32 passes on
-// the CTA path: the 2048-potential batch (93k levels) is fastest at 8192, the
-// 256-potential bump batch (14k levels) at 2048, the 64-Morse batch (3.4k
-// levels) at 1024-1536.  With the fallback levels and the psi zeroing on the
-// long levels' stream the 2048-potential batch measured 28.6 / 27.4 / 27.2 /
-// 27.3 ms a step at 6144 / 8192 / 10240 / 12288 points (flat from 8192 up).
+// Windows longer than a threshold take a CTA per level, the others a warp.  A
+// warp per level costs the fewest instructions (no barriers, one scan), but a
+// level's march is then 32 threads' and a batch of few levels leaves the GPU
+// idle, so the threshold falls with the number of levels.
 // DevBatch::long_window > 0 overrides it.
-constexpr int kLongWindow = 8192;
-constexpr int kLongWindowLevels = 60000;
+constexpr int kLongWindow = 65536;
+constexpr int kLongWindowLevels = 45000;
 constexpr int kMinLongWindow = 1024;
-// windows above this many points (and up to the long-window threshold) can
-// run their double-float passes one warp per level, after the lane FP32
-// refinement (DevBatch::mid_window > 0).  Off by default: on the
-// 2048-potential batch the warp passes (three marches of a chunked pass per
-// point) cost as much as the lane passes they replace (9 against 10 ms), and
-// the step was not shorter at thresholds of 1024 or 4096 points.
-constexpr int kMidWindow = -1;
 
 __host__ __device__ __forceinline__ int default_long_window(int total_levels) {
     int w = kMinLongWindow;
@@ -42,11 +25,26 @@ __host__ __device__ __forceinline__ int default_long_window(int total_levels) {
     return w;
 }
 
-// the level runs its double-float passes on a group of warps (CTA or warp
-// per level), not on a lane
-__device__ __forceinline__ bool is_long(const LevelWork& w) {
-    return (w.status & (EPSCU_STATUS_LONG | EPSCU_STATUS_MID)) != 0;
+// The threshold of the fragile levels' CTA passes (fragile.cu), which cost ~3x
+// the point-updates of a lane's but cut its latency ~80x: 8192 points at
+// >= ~9e4 levels, proportionally less below, never under 1024.
+constexpr int kFragileLongWindow = 8192;
+constexpr int kFragileLongLevels = 60000;
+constexpr int kFragileMinLongWindow = 1024;
+
+__host__ __device__ __forceinline__ int default_fragile_window(int total_levels) {
+    int w = kFragileMinLongWindow;
+    while (w < kFragileLongWindow && (long long)w * kFragileLongLevels < (long long)kFragileLongWindow * total_levels)
+        w <<= 1;
+    return w;
 }
+
+// Levels that share the scan's bracket with a neighbour, or whose brackets show
+// them this close to one (Hartree), are fragile (fragile.cu).
+constexpr double kFragileGap = 2e-5;
+
+// the level's final passes ran on a CTA
+__device__ __forceinline__ bool is_long(const LevelWork& w) { return (w.status & EPSCU_STATUS_LONG) != 0; }
 
 // match points stay inside the level's window, off its two end points
 __device__ __forceinline__ int clamp_k(const LevelWork& w, int k) { return max(w.j0 + 1, min(k, w.j1 - 1)); }
@@ -94,7 +92,7 @@ __device__ __forceinline__ bool redo_norm(const LevelWork& w, const PassDF& r) {
 }
 
 // The norm passes store psi-hat = (h + l) 2^X in the 8 bytes of each window
-// point of the level's row as a tagged float pair for scale_psi: X = 64 r + x
+// point of the level's row as a tagged float pair: X = 64 r + x
 // with x in [-32, 31], the pair (h 2^x, l 2^x) in floats, and r in the five
 // low bits of the second float (which only cost l bits 2^-43 below h).  X can
 // reach hundreds (a window edge deep in a steep wall lies far below the peak);
@@ -111,10 +109,14 @@ __device__ __forceinline__ PsiTag psi_tag(int X) {
     return {fpow2(X - 64 * r), r};
 }
 
-__device__ __forceinline__ void store_psi_pair(double* __restrict__ row, int i, dfl psi, PsiTag t) {
+__device__ __forceinline__ float2 psi_pair(dfl psi, PsiTag t) {
     const float l = __fmul_rn(psi.l, t.sc);
     const uint32_t lt = (__float_as_uint(l) & ~31u) | ((uint32_t)t.r & 31u);
-    reinterpret_cast<float2*>(row)[i] = make_float2(__fmul_rn(psi.h, t.sc), __uint_as_float(lt));
+    return make_float2(__fmul_rn(psi.h, t.sc), __uint_as_float(lt));
+}
+
+__device__ __forceinline__ void store_psi_pair(double* __restrict__ row, int i, dfl psi, PsiTag t) {
+    reinterpret_cast<float2*>(row)[i] = psi_pair(psi, t);
 }
 
 // the stored pair back: (h, l) and the tag r (psi-hat = (h + l) 2^(64 r))
@@ -124,8 +126,8 @@ __device__ __forceinline__ dfl load_psi_pair(float2 v, int& r) {
     return {v.x, __uint_as_float(lt & ~31u)};
 }
 
-// the level's psi row for the fused norm/write, or nullptr (no psi requested,
-// or the psi buffer overflowed: the level setup raised the capacity error)
+// the level's psi row, or nullptr (no psi requested, or the psi buffer
+// overflowed: the level setup raised the capacity error)
 __device__ __forceinline__ double* psi_row(const DevBatch& b, const PotMeta& m, const LevelWork& w) {
     if (!b.psi || b.hdr->error) return nullptr;
     return b.psi + m.psi_off + (int64_t)(w.v - b.min_level) * m.N;

@@ -11,12 +11,12 @@
 //   potentials the FP32 scan on every 16th trial energy, then a count round
 //   inside the cells where the counts change) -> level set-up + brackets
 //   plain : bisect64 -> norm64 -> twist64 -> write64            (native FP64)
-//   fast  : window, then two branches on two streams (graph fork/join):
-//             lane levels: refine32 -> newton_df -> norm_df
-//             long levels: refine_long -> norm_long, then (after newton_df)
-//                          the fallback levels' refinement and norm -> zero_psi
-//           -> twist_long -> scale_psi   (FP32, then compensated FP32 with
-//           FP64 matching and norm integral; the norm passes store psi-hat)
+//   fast  : window, order, then two branches on two streams (graph
+//           fork/join): levels<8> (a CTA per long level) and levels<1> (a
+//           warp per level), each taking a level through its FP32 passes, its
+//           double-float passes (FP64 matching and norm integral) and its psi
+//           row, then repair; beside them the fragile levels (fragile,
+//           fragile_repair)
 //   -> gather into the caller's layout.
 #include <cuda_runtime.h>
 
@@ -61,7 +61,7 @@ struct DevBuf {
     size_t cap = 0;
 };
 
-constexpr int kStageEvents = 12;  // 0-6 stages, 6-7 autotune, 8-9 around refine_long, 10-11 around zero_psi
+constexpr int kStageEvents = 10;  // 0-6 stages, 6-7 autotune, 8-9 around the level kernels
 
 }  // namespace
 
@@ -71,8 +71,8 @@ struct epscu_ctx {
     int device = 0;
     int sm_count = 0;
     cudaStream_t stream = nullptr;
-    cudaStream_t stream2 = nullptr;  // the long levels' branch of the fast pipeline
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_newton = nullptr;
+    cudaStream_t stream2 = nullptr;  // the fragile levels' branch of the fast pipeline
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     size_t block = size_t(64) << 20;
     std::map<std::string, DevBuf> bufs;
     std::map<std::string, std::pair<void*, size_t>> pinned;
@@ -111,7 +111,6 @@ struct epscu_ctx {
         if (ev_out) cudaEventDestroy(ev_out);
         if (ev_fork) cudaEventDestroy(ev_fork);
         if (ev_join) cudaEventDestroy(ev_join);
-        if (ev_newton) cudaEventDestroy(ev_newton);
         if (stream2) cudaStreamDestroy(stream2);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -241,13 +240,13 @@ epscu_status epscu_create(int32_t device_ordinal, epscu_ctx** out) {
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_out, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->ev_newton, cudaEventDisableTiming);
     if (e != cudaSuccess) {
         delete c;
         return fail(EPSCU_ERR_CUDA, std::string("context set-up: ") + cudaGetErrorString(e));
     }
     c->sm_count = p.multiProcessorCount;
     scan32_set_attributes();
+    levels_set_attributes();
     *out = c;
     return EPSCU_OK;
 }
@@ -332,58 +331,31 @@ void enqueue_pipeline(epscu_ctx* ctx, const DevBatch& b, int method, bool want_p
         if (want_psi) launch_write64(b, ctx->sm_count, s);
     } else {
         launch_window(b, ctx->sm_count, s);
+        launch_order_levels(b, ctx->sm_count, s);
         if (!stage_events) {
-            // the long levels (one CTA each), the middle levels (FP32 on lanes,
-            // then one warp each) and the lane levels are disjoint: the CTA
-            // branch runs beside the other two, filling the SMs the per-level
-            // kernels leave idle as they drain.  The psi rows are zeroed
-            // outside the level windows at the end of that branch, an HBM
-            // stream beside the compute-bound lane kernels (the norm passes
-            // write only inside the windows, so they need not wait for it;
-            // zeroing first held back the long levels' refinement: measured
-            // 29.6 against 28.7 ms a step on the 2048-potential batch).  The
-            // levels newton_df could not settle take their refinement and
-            // norm pass on CTAs in that branch too, once newton_df is done,
-            // so norm_df need not wait for them (28.7 -> 27.7 ms)
+            // the fragile levels, whose lane marches take longest, beside all
+            // others
             cudaEventRecord(ctx->ev_fork, s);
             cudaStreamWaitEvent(ctx->stream2, ctx->ev_fork, 0);
-            launch_refine32(b, ctx->sm_count, s);
-            launch_refine_long(b, ctx->sm_count, ctx->stream2);
-            launch_norm_long(b, ctx->sm_count, ctx->stream2);
-            launch_refine_mid(b, ctx->sm_count, s);
-            launch_newton_df(b, ctx->sm_count, s);
-            cudaEventRecord(ctx->ev_newton, s);
-            cudaStreamWaitEvent(ctx->stream2, ctx->ev_newton, 0);
-            launch_fallback_long(b, ctx->sm_count, ctx->stream2);
-            launch_norm_fallback(b, ctx->sm_count, ctx->stream2);
-            if (want_psi) launch_zero_psi(b, ctx->sm_count, ctx->stream2);
+            launch_fragile(b, ctx->sm_count, ctx->stream2);
+            launch_fragile_repair(b, ctx->sm_count, ctx->stream2);
             cudaEventRecord(ctx->ev_join, ctx->stream2);
-            launch_norm_mid(b, ctx->sm_count, s);
-            launch_norm_df(b, ctx->sm_count, s);
+            launch_long_levels(b, ctx->sm_count, s);
+            launch_warp_levels(b, ctx->sm_count, s);
+            launch_repair(b, ctx->sm_count, s);
             cudaStreamWaitEvent(s, ctx->ev_join, 0);
-            launch_twist_long(b, ctx->sm_count, s);
         } else {
             // stage timing: one stream, stages in sequence
-            launch_refine32(b, ctx->sm_count, s);
             rec(8);
-            launch_refine_long(b, ctx->sm_count, s);
+            launch_long_levels(b, ctx->sm_count, s);
+            launch_warp_levels(b, ctx->sm_count, s);
             rec(9);
             rec(3);
-            launch_refine_mid(b, ctx->sm_count, s);
-            launch_newton_df(b, ctx->sm_count, s);
-            launch_fallback_long(b, ctx->sm_count, s);
-            launch_norm_fallback(b, ctx->sm_count, s);
-            rec(10);
-            if (want_psi) launch_zero_psi(b, ctx->sm_count, s);
-            rec(11);
-            launch_norm_mid(b, ctx->sm_count, s);
-            launch_norm_df(b, ctx->sm_count, s);
-            launch_norm_long(b, ctx->sm_count, s);
-            launch_twist_long(b, ctx->sm_count, s);
+            launch_repair(b, ctx->sm_count, s);
+            launch_fragile(b, ctx->sm_count, s);
+            launch_fragile_repair(b, ctx->sm_count, s);
         }
         rec(4);
-        // rows written unnormalised by norm_df / norm_long / twist_long
-        if (want_psi) launch_scale_psi(b, ctx->sm_count, s);
     }
     rec(5);
 }
@@ -499,7 +471,8 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
     b.order = (int32_t*)ctx->get("order", sizeof(int32_t) * n, &ce);
     b.scan_win = nullptr;
     b.long_list = nullptr;
-    b.mid_list = nullptr;
+    b.warp_list = nullptr;
+    b.fragile_list = b.fragile_long = b.fragile_fall = b.fragile_twist = nullptr;
     b.bis_list = nullptr;
     b.bis_n = nullptr;
     b.bis_items = nullptr;
@@ -512,8 +485,14 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
         if (!b.Mpre || !b.Bmin) return fail(EPSCU_ERR_NOMEM, "device arena (window bounds)");
         b.long_list = (int32_t*)ctx->get("long_list", sizeof(int32_t) * lv, &ce);
         if (!b.long_list) return fail(EPSCU_ERR_NOMEM, "device arena (long list)");
-        b.mid_list = (int32_t*)ctx->get("mid_list", sizeof(int32_t) * lv, &ce);
-        if (!b.mid_list) return fail(EPSCU_ERR_NOMEM, "device arena (middle list)");
+        b.warp_list = (int32_t*)ctx->get("warp_list", sizeof(int32_t) * lv, &ce);
+        if (!b.warp_list) return fail(EPSCU_ERR_NOMEM, "device arena (warp list)");
+        b.fragile_list = (int32_t*)ctx->get("fragile_list", sizeof(int32_t) * lv, &ce);
+        b.fragile_long = (int32_t*)ctx->get("fragile_long", sizeof(int32_t) * lv, &ce);
+        b.fragile_fall = (int32_t*)ctx->get("fragile_fall", sizeof(int32_t) * lv, &ce);
+        b.fragile_twist = (int32_t*)ctx->get("fragile_twist", sizeof(int32_t) * b.max_twist, &ce);
+        if (!b.fragile_list || !b.fragile_long || !b.fragile_fall || !b.fragile_twist)
+            return fail(EPSCU_ERR_NOMEM, "device arena (fragile levels)");
         const size_t nb = (size_t)(batch->n_trial + kScanWinBlock - 1) / kScanWinBlock;
         b.scan_win = (int2*)ctx->get("scan_win", sizeof(int2) * (size_t)n * nb, &ce);
         if (!b.scan_win) return fail(EPSCU_ERR_NOMEM, "device arena (scan windows)");
@@ -554,7 +533,6 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
     b.tol = opts.tol;
     b.long_window = opts.long_window > 0 ? opts.long_window : 0;  // 0: chosen from the level count
     b.wait_polls = opts.wait_polls;  // 0: the default bound; < 0: the failure self-test
-    b.mid_window = opts.mid_window;  // 0: the default middle-tier threshold; < 0: no middle tier
     b.max_iter = opts.max_iter > 0 ? opts.max_iter : 0;            // 0: the default caps
     b.psi = nullptr;
     b.psi_capacity = 0;
@@ -639,8 +617,7 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
                   (void*)o_e, (void*)o_nt, (void*)o_no, (void*)o_nd, (void*)o_st, (void*)o_err,
                   (long long)b.psi_capacity, method, cap, shape.threads, shape.tile, shape.stages, opts.tol,
                   (void*)s);  // s is the context's own stream
-    keybuf_extra = std::to_string(b.long_window) + "|" + std::to_string(b.mid_window) + "|" +
-                   std::to_string(b.wait_polls) + "|" + std::to_string(b.max_iter);
+    keybuf_extra = std::to_string(b.long_window) + "|" + std::to_string(b.wait_polls) + "|" + std::to_string(b.max_iter);
     const std::string gkey = std::string(keybuf) + "|" + std::to_string(total_points) + "|" + keybuf_extra;
 
     auto enqueue_inputs = [&]() -> cudaError_t {
@@ -763,10 +740,7 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
         }
         st.ms_write = el(4, 5);
         st.ms_total = el(0, 6);
-        if (method == EPSCU_METHOD_FAST_FP32C) {
-            st.ms_refine_long = el(8, 9);
-            st.ms_zero_psi = el(10, 11);
-        }
+        if (method == EPSCU_METHOD_FAST_FP32C) st.ms_refine_long = el(8, 9);
     } else {
         cudaEventElapsedTime(&ms, ctx->ev[0], ctx->ev[6]);
         st.ms_total = ms;
@@ -782,21 +756,16 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
     // the windowed FP32 scan counts what it did; the FP64 scan covers [i0, i1]
     st.scan_point_updates = hh->scan_updates > 0 ? (int64_t)hh->scan_updates : scan_pts;
     st.n_levels = nlev;
-    st.fallbacks = hh->fallbacks;
-    st.twist_searches = hh->n_twist;
+    st.fallbacks = hh->fallbacks + hh->n_fragile_fall;
+    st.twist_searches = hh->n_twist + hh->n_fragile_twist;
     st.norm_redos = hh->n_redo;
     const bool psi_on = want_psi || keep_psi || (alloc_psi && b.psi);
     st.psi_bytes = psi_on ? psi_total * 8 : 0;
     // plain: prepare, scan64, level/unit setup, bracket, bisect64, norm64,
-    // twist64, gather (+ write64); fast: prepare, scan window, scan32, level/unit
-    // setup, bracket, window, refine32, refine_long, newton_df, fallback
-    // (refine_long over the fallback list), its norm (norm_long over the
-    // fallback list), norm_df, norm_long, twist_long, gather (+ refine_mid,
-    // norm_mid with the middle tier; + zero_psi, scale_psi)
-    const bool psi_kernels = psi_on;
-    const bool mid_on = b.mid_list && (b.mid_window != 0 ? b.mid_window : kMidWindow) > 0;
-    st.kernel_launches = method == EPSCU_METHOD_FAST_FP32C ? 16 + (mid_on ? 2 : 0) + (psi_kernels ? 2 : 0)
-                                                           : 9 + (psi_kernels ? 1 : 0);
+    // twist64, gather (+ write64); fast: prepare, scan window, scan32, level
+    // setup, bracket, window, order, the two level kernels, repair, the two
+    // fragile kernels, gather
+    st.kernel_launches = method == EPSCU_METHOD_FAST_FP32C ? 13 : 9 + (psi_on ? 1 : 0);
     if (b.bis_list) {  // the plan + count rounds after the coarse scan32
         for (int W = kBisectCoarse; W > 1; W /= (W < kBisectSplit ? W : kBisectSplit)) st.kernel_launches += 2;
     }
@@ -864,13 +833,14 @@ extern "C" epscu_status epscu_adjoint(epscu_ctx* ctx, const double* dL_dE, doubl
         b.psi = psi;
         b.psi_capacity = ctx->last_psi_total;
         // the writer of the solve's own method (its norm constants belong to it)
-        const int qid = ctx->last_method == EPSCU_METHOD_FAST_FP32C ? kQWriteDF : kQWrite64;
-        EPSCU_CU(cudaMemsetAsync(&b.hdr->queue[qid], 0, sizeof(int32_t), s));
         if (ctx->last_method == EPSCU_METHOD_FAST_FP32C) {
-            launch_zero_psi(b, ctx->sm_count, s);  // write_long writes only the windows
-            launch_write_df(b, ctx->sm_count, s);
-            launch_write_long(b, ctx->sm_count, s);
+            EPSCU_CU(cudaMemsetAsync(&b.hdr->queue[kQWarpRewrite], 0, sizeof(int32_t), s));
+            EPSCU_CU(cudaMemsetAsync(&b.hdr->queue[kQLongRewrite], 0, sizeof(int32_t), s));
+            EPSCU_CU(cudaMemsetAsync(&b.hdr->queue[kQFragileRewrite], 0, sizeof(int32_t), s));
+            launch_rewrite(b, ctx->sm_count, s);
+            launch_fragile_rewrite(b, ctx->sm_count, s);
         } else {
+            EPSCU_CU(cudaMemsetAsync(&b.hdr->queue[kQWrite64], 0, sizeof(int32_t), s));
             launch_write64(b, ctx->sm_count, s);
         }
     }

@@ -1,58 +1,34 @@
-// longwin.cu -- the fast method's per-level passes on groups of warps.
+// fragile.cu -- levels whose results the last bits of their passes decide.
 //
-// A level whose window is long (a long grid: the 2^20-point Morse has windows
-// of 10^5 - 4.7 10^5 points; on the mixed batch every window above a few
-// thousand points) cannot be marched by one lane: a pass would cost ~10^4 -
-// 10^6 dependent steps of latency while most of the GPU idles.  Such a level
-// takes a group of NW warps instead: the whole CTA (NW = 8) for the longest
-// windows, or one warp (NW = 1) for the middle tier.  Each side of a pass
-// (outward from j0 to the match point k, inward from j1 to k) is split into
-// one contiguous chunk per thread of the group and the double-float
-// difference-form recurrence
-//     D' = D + T (D - 12 A),   A' = A + (T A + D')
-// runs in three phases:
+//  * On grids that do not resolve the wavelength (k_max h > 1:
+//    EPSCU_LEVEL_UNDER_RESOLVED) counts and energies of the discrete problem
+//    are exact, but a level's matching function can have a pole within a
+//    rounding error of its root: the node count of its shooting solution, and
+//    now and then which of two close roots an iteration ends in, hang on the
+//    rounding.
+//  * Levels close to a neighbour (kFragileGap): psi mixes with the neighbour's
+//    by the energy's resolution over the gap, 1e-13 / 1e-5 = 1e-8.
+// These levels (12% and ~0.2% of the 2048-potential mixed batch) keep passes of
+// their own, whose order of operations their results depend on: two lanes
+// per level marching its window from both ends (lane32.cuh, lanedf.cuh), a CTA
+// per level for windows above a threshold (the passes below), the twist-index
+// search for levels whose final pass disagrees.  All other levels take
+// levelpass.cu's.
+//
+// The CTA passes split each side of a pass (outward from j0 to the match point
+// k, inward from j1 to k) into one contiguous chunk per thread:
 //   1. every thread marches the two unit states (A, D) = (1, 0) and (0, 1)
-//      through its chunk: the step is linear in (A, D), so these are the
-//      columns of the chunk's 2x2 transfer matrix (with the product of 1/f
-//      over the chunk for the passes that need psi);
-//   2. a parallel prefix scan of the transfer matrices -- Hillis-Steele over
-//      the 32 lanes of each warp with shuffles, then over the group's warps
-//      through shared memory -- gives the exact starting state and scale of
-//      every chunk;
+//      through its chunk (the step D' = D + T (D - 12 A), A' = A + (T A + D')
+//      is linear): the chunk's 2x2 transfer matrix, and the product of 1/f
+//      over the chunk for the passes that need psi;
+//   2. a prefix scan of the matrices, Hillis-Steele over the lanes with
+//      shuffles, then over the warps through shared memory, gives every
+//      chunk's exact starting state and scale (products renormalised by powers
+//      of two, exponents in ints);
 //   3. every thread re-runs its chunk from that state: node counts, the sum
-//      of psi^2, the peak of |psi| or the psi write, reduced over the group.
-// A pass costs about three serial marches of point-updates, spread over the
-// group.  The matrices span exponential growth, so every product is
-// renormalised by a power of two with the exponent carried in an int; the
-// physical solution is the growing one on both sides (each side runs from a
-// forbidden region towards the match point at the peak of |psi|), so a
-// product applied to the starting state loses nothing to the discarded
-// subdominant solution.
-//
-// FP64 runs once per pass, in the group's thread 0 (the leader): the sums are
-// reduced over the warps in FP32 (FP32 passes) or double-float (double-float
-// passes) with their binary exponents aligned, and the leader forms the
-// side's sum in FP64, the matching function gamma_k, the psi^2 sum and the
-// Cooley step, and hands the pass's result to the group through shared
-// memory.  (Every thread doing that FP64 work kept the FP64 pipe, 1/62 of the
-// FP32 rate on GB300, busy for a large part of a pass on windows of a few
-// thousand points per CTA.)
-//
-// Kernels (one group per level, levels taken from a device queue over a list
-// the window kernel fills; the lane-per-level kernels skip these levels):
-//   refine_long : from the scan bracket, FP32 passes (the same three phases
-//                 in FP32, long_side32) to a Newton step of 3e-8, then double-float
-//                 state-only Newton to 1e-12 (replaces refine32 + newton_df);
-//                 run again over the levels newton_df could not settle (the
-//                 fallback: any window length, full double-float passes from
-//                 the scan bracket widened by one trial spacing), and over
-//                 the middle list from the lane FP32 refinement's result;
-//   norm_long   : the norm pass and its match-point candidates (as norm_df),
-//                 storing psi-hat as tagged float pairs for scale_psi; run
-//                 over the long list and over the fallback list;
-//   twist_long  : the twist-index search for the levels the norm passes flag;
-//   write_long  : psi from the final constants (the adjoint's recompute path;
-//                 the long, middle and fallback lists).
+//      of psi^2, the peak of |psi| or the psi write, reduced over the CTA.
+// FP64 runs once per pass, in the CTA's thread 0 (the leader), which hands the
+// pass's result on through shared memory.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -60,7 +36,10 @@
 #include "common.cuh"
 #include "dfloat.cuh"
 #include "dfpass.cuh"
+#include "lane32.cuh"
+#include "lanedf.cuh"
 #include "launch.h"
+#include "psirow.cuh"
 
 namespace epscu {
 
@@ -71,6 +50,9 @@ namespace {
 constexpr int kLongThreads = 256;
 constexpr int kLongWarps = kLongThreads / 32;
 constexpr int kLongCtasPerSm = 2;
+// first of this file's rows of the twist scratch (levelpass.cu's CTAs, which may
+// run at the same time, use the first ones)
+constexpr int kFragileScratch = 2048;
 
 // [[a, b], [c, d]] 2^e acting on the column (A, D)
 struct Mat2 {
@@ -154,48 +136,29 @@ __device__ __forceinline__ void df_step(dfl T, dfl& A, dfl& D) {
 }
 
 // ---------------------------------------------------------------- groups
-// A level's passes run on a group of NW warps (NW = 8: the whole CTA of
-// kLongThreads; NW = 1: one warp, kLongThreads / 32 groups per CTA).  The
-// group's thread 0 is its leader.
-template <int NW>
+// A level's passes run on a CTA; its thread 0 is the leader.
 struct Grp {
-    static constexpr int kThreads = 32 * NW;
-    // thread in the group, lane, warp in the group, group in the CTA (read
-    // from threadIdx each time: nothing held in registers)
-    __device__ __forceinline__ int t() const { return (int)(threadIdx.x % kThreads); }
+    static constexpr int kThreads = kLongThreads;
+    __device__ __forceinline__ int t() const { return (int)threadIdx.x; }
     __device__ __forceinline__ int lane() const { return (int)(threadIdx.x & 31); }
-    __device__ __forceinline__ int warp() const { return (int)((threadIdx.x % kThreads) >> 5); }
-    __device__ __forceinline__ int g() const { return (int)(threadIdx.x / kThreads); }
-    __device__ __forceinline__ bool leader() const { return t() == 0; }
+    __device__ __forceinline__ int warp() const { return (int)(threadIdx.x >> 5); }
+    __device__ __forceinline__ bool leader() const { return threadIdx.x == 0; }
 };
 
-template <int NW>
-__device__ __forceinline__ void gsync() {
-    static_assert(NW == 1 || NW == kLongWarps, "a group is one warp or the whole CTA");
-    if constexpr (NW == 1) __syncwarp();
-    else __syncthreads();
-}
-
-// the leader's value to the whole group (slot: the group's shared word)
-template <int NW>
-__device__ __forceinline__ int grp_bcast(const Grp<NW>& G, int v, int& slot) {
-    if constexpr (NW == 1) {
-        return __shfl_sync(0xffffffffu, v, 0);
-    } else {
-        if (G.leader()) slot = v;
-        __syncthreads();
-        const int r = slot;
-        __syncthreads();  // every thread has read the slot
-        return r;
-    }
+// the leader's value to the whole CTA (slot: a shared word)
+__device__ __forceinline__ int grp_bcast(const Grp& G, int v, int& slot) {
+    if (G.leader()) slot = v;
+    __syncthreads();
+    const int r = slot;
+    __syncthreads();  // every thread has read the slot
+    return r;
 }
 
 // the next entry of a device queue for the group
-template <int NW>
-__device__ __forceinline__ int grp_next(const Grp<NW>& G, int* queue, int& slot) {
+__device__ __forceinline__ int grp_next(const Grp& G, int* queue, int& slot) {
     int q = 0;
     if (G.leader()) q = atomicAdd(queue, 1);
-    return grp_bcast<NW>(G, q, slot);
+    return grp_bcast(G, q, slot);
 }
 
 // A non-negative sum (h + l) 2^e in double-float, and its warp-wide total:
@@ -260,15 +223,14 @@ __device__ __forceinline__ double dfe_to_double(DfE x) {
 }
 
 // ------------------------------------------------------- double-float sides
-template <int NW>
 struct SharedDF {
-    Mat2 wtot[NW], wpre[NW];
-    Scal qtot[NW], qpre[NW];
-    int nodes[NW];
-    DfE s[NW];  // warp partial sums of psi-hat^2, absolute exponents
-    int pk_L[NW], pk_s[NW];
-    double gb[NW];  // MODE 5: warp minima of |gamma| and their points
-    int gk[NW];
+    Mat2 wtot[kLongWarps], wpre[kLongWarps];
+    Scal qtot[kLongWarps], qpre[kLongWarps];
+    int nodes[kLongWarps];
+    DfE s[kLongWarps];  // warp partial sums of psi-hat^2, absolute exponents
+    int pk_L[kLongWarps], pk_s[kLongWarps];
+    double gb[kLongWarps];  // MODE 5: warp minima of |gamma| and their points
+    int gk[kLongWarps];
     // the side's final state (written by the thread holding the last chunk)
     dfl A, D, q;
     int eA, eQ;
@@ -305,15 +267,15 @@ struct TwistIO {
     int k;              //   and its point
 };
 
-template <int NW, int MODE>
-__device__ LongSide<MODE> long_side(const Grp<NW>& G, const float2* __restrict__ Wf, dfl aE, int from, int to,
-                                    int dir, double* __restrict__ out, double L, int Xk, SharedDF<NW>& sh,
+template <int MODE>
+__device__ LongSide<MODE> long_side(const Grp& G, const float2* __restrict__ Wf, dfl aE, int from, int to,
+                                    int dir, double* __restrict__ out, double L, int Xk, SharedDF& sh,
                                     TwistIO* tw = nullptr) {
     // MODE 0: state, 1: + sums/peak, 2: + psi write, 3: MODE 1 + unnormalised
     // psi-hat written in the absolute scale, 4/5: twist sweeps (state)
     constexpr bool kPsi = MODE == 1 || MODE == 2 || MODE == 3;
     constexpr bool kSums = MODE == 1 || MODE == 3;
-    constexpr int kT = Grp<NW>::kThreads;
+    constexpr int kT = Grp::kThreads;
     const int tid = G.t(), lane = G.lane(), warp = G.warp();
     const int nsteps = (to - from) * dir;
     LongSide<MODE> res;
@@ -377,33 +339,28 @@ __device__ LongSide<MODE> long_side(const Grp<NW>& G, const float2* __restrict__
     }
     Mat2 Mx = shfl_up_mat(M, 1);
     Scal Px = shfl_up_scal(P, 1);
-    if constexpr (NW > 1) {
-        if (lane == 31) {
-            sh.wtot[warp] = M;
-            sh.qtot[warp] = P;
+    if (lane == 31) {
+        sh.wtot[warp] = M;
+        sh.qtot[warp] = P;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        Mat2 acc = mat_identity();
+        Scal qa{{1.0f, 0.0f}, 0};
+        for (int w = 0; w < kLongWarps; ++w) {
+            sh.wpre[w] = acc;
+            sh.qpre[w] = qa;
+            acc = mat_mul(sh.wtot[w], acc);
+            if (kPsi) qa = scal_mul(sh.qtot[w], qa);
         }
-        gsync<NW>();
-        if (tid == 0) {
-            Mat2 acc = mat_identity();
-            Scal qa{{1.0f, 0.0f}, 0};
-            for (int w = 0; w < NW; ++w) {
-                sh.wpre[w] = acc;
-                sh.qpre[w] = qa;
-                acc = mat_mul(sh.wtot[w], acc);
-                if (kPsi) qa = scal_mul(sh.qtot[w], qa);
-            }
-        }
-        gsync<NW>();
-        if (lane == 0) {
-            Mx = sh.wpre[warp];
-            Px = sh.qpre[warp];
-        } else {
-            Mx = mat_mul(Mx, sh.wpre[warp]);
-            if (kPsi) Px = scal_mul(Px, sh.qpre[warp]);
-        }
-    } else if (lane == 0) {
-        Mx = mat_identity();
-        Px = {{1.0f, 0.0f}, 0};
+    }
+    __syncthreads();
+    if (lane == 0) {
+        Mx = sh.wpre[warp];
+        Px = sh.qpre[warp];
+    } else {
+        Mx = mat_mul(Mx, sh.wpre[warp]);
+        if (kPsi) Px = scal_mul(Px, sh.qpre[warp]);
     }
 
     // ---- phase 3: this chunk from its starting state (A, D) = Mx (1, 1)
@@ -550,7 +507,7 @@ __device__ LongSide<MODE> long_side(const Grp<NW>& G, const float2* __restrict__
             sh.gk[warp] = g_k;
         }
     }
-    gsync<NW>();
+    __syncthreads();
     if (G.leader()) {
         res.A = sh.A;
         res.D = sh.D;
@@ -560,7 +517,7 @@ __device__ LongSide<MODE> long_side(const Grp<NW>& G, const float2* __restrict__
         int nsum = 0;
         double Ssum = 0.0;
         int pL = -(1 << 30), ps = 0x7fffffff;
-        for (int w = 0; w < NW; ++w) {
+        for (int w = 0; w < kLongWarps; ++w) {
             nsum += sh.nodes[w];
             if (kSums) {
                 // the warp's sum in the side's final scale
@@ -582,7 +539,7 @@ __device__ LongSide<MODE> long_side(const Grp<NW>& G, const float2* __restrict__
         // every thread of the group takes the search's result
         double gb = INFINITY;
         int gk = 0x7fffffff;
-        for (int w = 0; w < NW; ++w)
+        for (int w = 0; w < kLongWarps; ++w)
             if (sh.gb[w] < gb || (sh.gb[w] == gb && sh.gk[w] < gk)) {
                 gb = sh.gb[w];
                 gk = sh.gk[w];
@@ -599,16 +556,16 @@ __device__ LongSide<MODE> long_side(const Grp<NW>& G, const float2* __restrict__
 // leader turns the two sides into the Cooley correction, the count, the sum
 // and the peak, and hands the result to the group.  MODE 3 also stores the
 // unnormalised psi-hat of the window in row (if not null).
-template <int NW, int MODE>
-__device__ __forceinline__ PassDF long_pass(const Grp<NW>& G, const PotMeta& m, const LevelWork& w,
+template <int MODE>
+__device__ __forceinline__ PassDF long_pass(const Grp& G, const PotMeta& m, const LevelWork& w,
                                             const float2* __restrict__ Wf, const double* __restrict__ W64, double E,
-                                            int k, double sum_fallback, SharedDF<NW>& sh,
+                                            int k, double sum_fallback, SharedDF& sh,
                                             double* __restrict__ row = nullptr) {
     if (G.leader()) sh.aE = energy_df(m, E);
-    gsync<NW>();
+    __syncthreads();
     const dfl aE = sh.aE;
-    const LongSide<MODE> o = long_side<NW, MODE>(G, Wf, aE, w.j0, k, +1, row, 0.0, 0, sh);
-    const LongSide<MODE> in = long_side<NW, MODE>(G, Wf, aE, w.j1, k, -1, row, 0.0, 0, sh);
+    const LongSide<MODE> o = long_side<MODE>(G, Wf, aE, w.j0, k, +1, row, 0.0, 0, sh);
+    const LongSide<MODE> in = long_side<MODE>(G, Wf, aE, w.j1, k, -1, row, 0.0, 0, sh);
     if (G.leader()) {
         const double Tk = __dsub_rn(__dmul_rn(m.a, E), __ldg(W64 + k));
         const double fk = 1.0 + Tk;
@@ -640,7 +597,7 @@ __device__ __forceinline__ PassDF long_pass(const Grp<NW>& G, const PotMeta& m, 
         r.dE = r.gamma * fk * fk / (12.0 * m.a * r.sum);
         sh.res = r;
     }
-    gsync<NW>();
+    __syncthreads();
     return sh.res;
 }
 
@@ -711,14 +668,13 @@ __device__ __forceinline__ Scalf shfl_up_scalf(const Scalf& s, int o) {
     return {__shfl_up_sync(0xffffffffu, s.v, o), __shfl_up_sync(0xffffffffu, s.e, o)};
 }
 
-template <int NW>
 struct Shared32 {
-    Mat2f wtot[NW], wpre[NW];
-    Scalf ftot[NW], fpre[NW];
+    Mat2f wtot[kLongWarps], wpre[kLongWarps];
+    Scalf ftot[kLongWarps], fpre[kLongWarps];
     Scalf fall;  // product of f^2 over the side
-    int nodes[NW];
-    FE s[NW];  // warp partial sums, absolute exponents
-    int pk_L[NW], pk_s[NW];
+    int nodes[kLongWarps];
+    FE s[kLongWarps];  // warp partial sums, absolute exponents
+    int pk_L[kLongWarps], pk_s[kLongWarps];
     float A, D;  // the side's final state (thread holding the last chunk)
     int eA;
     // the leader's broadcasts: a E as a float pair and the pass result
@@ -742,10 +698,9 @@ struct LongSide32 {
 // them, phase 3 re-runs the chunk from its exact start state; a chunk's S is
 // carried to the side's end by the product of F over the later chunks.  The
 // result is valid in the leader.
-template <int NW>
-__device__ LongSide32 long_side32(const Grp<NW>& G, const float2* __restrict__ Wf, float aEh, float aEl, int from,
-                                  int to, int dir, Shared32<NW>& sh) {
-    constexpr int kT = Grp<NW>::kThreads;
+__device__ LongSide32 long_side32(const Grp& G, const float2* __restrict__ Wf, float aEh, float aEl, int from,
+                                  int to, int dir, Shared32& sh) {
+    constexpr int kT = Grp::kThreads;
     const int tid = G.t(), lane = G.lane(), warp = G.warp();
     const int nsteps = (to - from) * dir;
     LongSide32 res;
@@ -811,32 +766,27 @@ __device__ LongSide32 long_side32(const Grp<NW>& G, const float2* __restrict__ W
     Mat2f Mx = shfl_up_matf(M, 1);
     Scalf Fin = F;  // f^2 over the chunks up to this thread's
     Scalf Fall;     // f^2 over the side
-    if constexpr (NW > 1) {
-        if (lane == 31) {
-            sh.wtot[warp] = M;
-            sh.ftot[warp] = F;
-        }
-        gsync<NW>();
-        if (tid == 0) {
-            Mat2f acc = {1.0f, 0.0f, 0.0f, 1.0f, 0};
-            Scalf fa{1.0f, 0};
-            for (int w = 0; w < NW; ++w) {
-                sh.wpre[w] = acc;
-                sh.fpre[w] = fa;
-                acc = matf_mul(sh.wtot[w], acc);
-                fa = scalf_mul(sh.ftot[w], fa);
-            }
-            sh.fall = fa;
-        }
-        gsync<NW>();
-        if (lane == 0) Mx = sh.wpre[warp];
-        else Mx = matf_mul(Mx, sh.wpre[warp]);
-        Fin = scalf_mul(F, sh.fpre[warp]);
-        Fall = sh.fall;
-    } else {
-        if (lane == 0) Mx = {1.0f, 0.0f, 0.0f, 1.0f, 0};
-        Fall = {__shfl_sync(0xffffffffu, F.v, 31), __shfl_sync(0xffffffffu, F.e, 31)};
+    if (lane == 31) {
+        sh.wtot[warp] = M;
+        sh.ftot[warp] = F;
     }
+    __syncthreads();
+    if (tid == 0) {
+        Mat2f acc = {1.0f, 0.0f, 0.0f, 1.0f, 0};
+        Scalf fa{1.0f, 0};
+        for (int w = 0; w < kLongWarps; ++w) {
+            sh.wpre[w] = acc;
+            sh.fpre[w] = fa;
+            acc = matf_mul(sh.wtot[w], acc);
+            fa = scalf_mul(sh.ftot[w], fa);
+        }
+        sh.fall = fa;
+    }
+    __syncthreads();
+    if (lane == 0) Mx = sh.wpre[warp];
+    else Mx = matf_mul(Mx, sh.wpre[warp]);
+    Fin = scalf_mul(F, sh.fpre[warp]);
+    Fall = sh.fall;
 
     // ---- phase 3: this chunk from its start state (A, D) = Mx (1, 1)
     float A = Mx.a + Mx.b, D = Mx.c + Mx.d;
@@ -913,7 +863,7 @@ __device__ LongSide32 long_side32(const Grp<NW>& G, const float2* __restrict__ W
         sh.pk_s[warp] = peak_s;
         sh.s[warp] = sw;
     }
-    gsync<NW>();
+    __syncthreads();
     if (G.leader()) {
         res.A = sh.A;
         res.D = sh.D;
@@ -921,7 +871,7 @@ __device__ LongSide32 long_side32(const Grp<NW>& G, const float2* __restrict__ W
         int nsum = 0;
         double Ssum = 0.0;
         int pL = -(1 << 30), ps = 0x7fffffff;
-        for (int w = 0; w < NW; ++w) {
+        for (int w = 0; w < kLongWarps; ++w) {
             nsum += sh.nodes[w];
             const FE s = sh.s[w];
             if (s.v > 0.0f) Ssum += (double)s.v * pow2(max(-1000, min(1000, s.e - 2 * res.eA)));
@@ -941,20 +891,19 @@ __device__ LongSide32 long_side32(const Grp<NW>& G, const float2* __restrict__ W
 // One FP32 pass at E with match point k (the group twin of the lane pass):
 // Cooley correction, count, sum and the peak of |psi| relative to psi_k,
 // formed by the leader and handed to the group.
-template <int NW>
-__device__ __forceinline__ PassDF long_pass32(const Grp<NW>& G, const PotMeta& m, const LevelWork& w,
+__device__ __forceinline__ PassDF long_pass32(const Grp& G, const PotMeta& m, const LevelWork& w,
                                               const float2* __restrict__ Wf, const double* __restrict__ W64,
-                                              double E, int k, Shared32<NW>& sh) {
+                                              double E, int k, Shared32& sh) {
     if (G.leader()) {
         const double aE = __dmul_rn(m.a, E);
         const float aEh = __double2float_rn(aE);
         sh.aEh = aEh;
         sh.aEl = __double2float_rn(aE - (double)aEh);
     }
-    gsync<NW>();
+    __syncthreads();
     const float aEh = sh.aEh, aEl = sh.aEl;
-    const LongSide32 o = long_side32<NW>(G, Wf, aEh, aEl, w.j0, k, +1, sh);
-    const LongSide32 in = long_side32<NW>(G, Wf, aEh, aEl, w.j1, k, -1, sh);
+    const LongSide32 o = long_side32(G, Wf, aEh, aEl, w.j0, k, +1, sh);
+    const LongSide32 in = long_side32(G, Wf, aEh, aEl, w.j1, k, -1, sh);
     if (G.leader()) {
         const double aE = __dmul_rn(m.a, E);
         const double Tk = aE - __ldg(W64 + k);
@@ -977,19 +926,18 @@ __device__ __forceinline__ PassDF long_pass32(const Grp<NW>& G, const PotMeta& m
         r.ex_out = r.ex_in = 0;
         sh.res = r;
     }
-    gsync<NW>();
+    __syncthreads();
     return sh.res;
 }
 
 // the host-mapped cancel flag, read by the leader and handed to the group
 // (threads that read it separately could see it change between their reads
 // and part at the next barrier)
-template <int NW>
-__device__ __forceinline__ bool grp_cancelled(const Grp<NW>& G, const DevBatch& b, int& slot) {
-    return grp_bcast<NW>(G, G.leader() && b.cancel && *b.cancel ? 1 : 0, slot) != 0;
+__device__ __forceinline__ bool grp_cancelled(const Grp& G, const DevBatch& b, int& slot) {
+    return grp_bcast(G, G.leader() && b.cancel && *b.cancel ? 1 : 0, slot) != 0;
 }
 
-// Levels on groups of warps, in up to three stages:
+// The refinement of a level, in up to three stages:
 //   1. FP32 passes (long_pass32): safeguarded Cooley-Newton with the count
 //      bracket, the match point moved to the peak of |psi|, until a Newton
 //      step of at most kTol32Long is taken (the energy after it is then far
@@ -1016,48 +964,61 @@ __device__ __forceinline__ bool grp_cancelled(const Grp<NW>& G, const DevBatch& 
 // double-float passes after it.)
 constexpr double kTol32Long = 3e-8;
 
-template <int NW>
-__global__ void __launch_bounds__(kLongThreads, kLongCtasPerSm) refine_long_kernel(DevBatch b, int mode, const int32_t* list,
-                                                                   const int32_t* list_len, int qid) {
-    constexpr int kG = kLongThreads / (32 * NW);
-    __shared__ SharedDF<NW> shd[kG];
-    __shared__ Shared32<NW> sh32s[kG];
-    const Grp<NW> G;
-    SharedDF<NW>& sh = shd[G.g()];
-    Shared32<NW>& sh32 = sh32s[G.g()];
-    const int n = min(*list_len, b.max_levels);  // filled on the device earlier in the solve
-    // levels from a device queue (a group takes the next as it finishes one)
-    for (;;) {
-        const int q = grp_next<NW>(G, &b.hdr->queue[qid], sh.word);
-        if (q >= n) break;
-        const int slot = list[q];
-        LevelWork w = b.levels[slot];
-        if (w.status & EPSCU_STATUS_NOTFOUND) continue;
-        if (grp_cancelled<NW>(G, b, sh.word)) {
-            if (G.leader()) b.levels[slot].status = w.status | EPSCU_STATUS_CANCELLED;
-            continue;
+__device__ __noinline__ void refine_cta(const Grp& G, const DevBatch& b, LevelWork& w, bool fallback, SharedDF& sh,
+                                        Shared32& sh32) {
+    const PotMeta m = b.meta[w.p];
+    const float2* Wf = b.Wf2 + m.offf;
+    const double* W = b.W64 + m.off;
+    double lo = w.lo, hi = w.hi, E = w.E, sum = 1.0;
+    int k = grp_bcast(G, G.leader() ? clamp_k(w, match_index(m, b.Msuf, E)) : 0, sh.word);
+    bool done = false;
+    int n_pass = 0, n_pass32 = 0;
+    if (!fallback) {
+        // ---- stage 1: FP32
+        bool moved_last = false, ok32 = false;
+        for (int it = 0, cap = refine_cap(b); it < cap; ++it) {
+            const PassDF r = long_pass32(G, m, w, Wf, W, E, k, sh32);
+            ++n_pass32;
+            sum = r.sum;
+            if (r.count > w.v) hi = E;
+            else lo = E;
+            if (r.peak_log2 >= 2 && !moved_last) {
+                k = clamp_k(w, r.peak_i);
+                moved_last = true;
+                continue;  // the same energy at the new match point
+            }
+            moved_last = false;
+            const double En = E + r.dE;
+            const bool near = r.nodes == w.v || (m.status & EPSCU_STATUS_UNDER);
+            if (near && isfinite(En) && En > lo && En < hi) {
+                E = En;
+                if (fabs(r.dE) <= kTol32Long) {
+                    ok32 = true;
+                    break;
+                }
+            } else {
+                E = 0.5 * (lo + hi);
+            }
+            if (hi - lo <= 2.0 * kTol32Long) {
+                E = 0.5 * (lo + hi);
+                ok32 = true;
+                break;
+            }
         }
-        const PotMeta m = b.meta[w.p];
-        const float2* Wf = b.Wf2 + m.offf;
-        const double* W = b.W64 + m.off;
-        double lo = w.lo, hi = w.hi, E = w.E, sum = 1.0;
-        int k = mode == 2 ? w.k : grp_bcast<NW>(G, G.leader() ? clamp_k(w, match_index(m, b.Msuf, E)) : 0, sh.word);
-        bool done = false;
-        int n_pass = 0, n_pass32 = 0;
-        if (mode == 2) {
-            // ---- stage 2 from the lane FP32 refinement (as newton_df): its sum
-            // psi~^2 is accurate to ~1e-4 on long windows, so one step is
-            // accepted from within 1e-10 and the norm pass corrects the rest
-            sum = w.norm_k_in;
-            double lo2 = w.lo - 1e-8, hi2 = w.hi + 1e-8;
+        // ---- stage 2: double-float state-only Newton (FP32 sum)
+        if (ok32) {
+            double lo2 = lo - 1e-8, hi2 = hi + 1e-8;
             for (int it = 0; it < 4 && !done; ++it) {
-                const PassDF r = long_pass<NW, 0>(G, m, w, Wf, W, E, k, sum, sh);
+                const PassDF r = long_pass<0>(G, m, w, Wf, W, E, k, sum, sh);
                 ++n_pass;
                 if (r.count > w.v) hi2 = fmin(hi2, E);
                 else lo2 = fmax(lo2, E);
                 const double En = E + r.dE;
                 if (!isfinite(En) || !(En >= lo2 && En <= hi2) || r.nodes != w.v) break;
-                done = fabs(r.dE) <= (it == 0 ? 1e-10 : 1e-12 * fmax(1.0, fabs(E)));
+                // the FP32 sum of the group pass is accurate to ~1e-6 (chunk
+                // sums of a few hundred terms), so one step from within 1e-8
+                // leaves ~1e-14: the first pass settles
+                done = fabs(r.dE) <= (it == 0 ? 1e-8 * fmax(1.0, fabs(E)) : 1e-12 * fmax(1.0, fabs(E)));
                 E = En;
             }
             if (done) {
@@ -1065,307 +1026,306 @@ __global__ void __launch_bounds__(kLongThreads, kLongCtasPerSm) refine_long_kern
                 hi = hi2;
             }
         }
-        if (mode == 0) {
-            // ---- stage 1: FP32
-            bool moved_last = false, ok32 = false;
-            for (int it = 0, cap = refine_cap(b); it < cap; ++it) {
-                const PassDF r = long_pass32<NW>(G, m, w, Wf, W, E, k, sh32);
-                ++n_pass32;
-                sum = r.sum;
-                if (r.count > w.v) hi = E;
-                else lo = E;
-                if (r.peak_log2 >= 2 && !moved_last) {
-                    k = clamp_k(w, r.peak_i);
-                    moved_last = true;
-                    continue;  // the same energy at the new match point
-                }
-                moved_last = false;
-                const double En = E + r.dE;
-                const bool near = r.nodes == w.v || (m.status & EPSCU_STATUS_UNDER);
-                if (near && isfinite(En) && En > lo && En < hi) {
-                    E = En;
-                    if (fabs(r.dE) <= kTol32Long) {
-                        ok32 = true;
-                        break;
-                    }
-                } else {
-                    E = 0.5 * (lo + hi);
-                }
-                if (hi - lo <= 2.0 * kTol32Long) {
-                    E = 0.5 * (lo + hi);
-                    ok32 = true;
-                    break;
-                }
+    }
+    if (!done) {
+        // ---- stage 3: the FP32 bracket may be off by its count errors:
+        // restart from the scan bracket widened by one trial spacing
+        lo = fmax(m.e_lo, w.lo0 - m.delta);
+        hi = fmin(m.e_cap, w.hi0 + m.delta);
+        if (!(E > lo && E < hi)) E = 0.5 * (lo + hi);
+        bool moved_last = false;
+        for (int it = 0, cap = fallback_cap(b); it < cap; ++it) {
+            const PassDF r = long_pass<1>(G, m, w, Wf, W, E, k, 1.0, sh);
+            ++n_pass;
+            sum = r.sum;
+            if (r.count > w.v) hi = E;
+            else lo = E;
+            if (r.peak_log2 >= 2 && !moved_last) {
+                k = clamp_k(w, r.peak_i);
+                moved_last = true;
+                continue;  // the same energy at the new match point
             }
-            // ---- stage 2: double-float state-only Newton (FP32 sum)
-            if (ok32) {
-                double lo2 = lo - 1e-8, hi2 = hi + 1e-8;
-                for (int it = 0; it < 4 && !done; ++it) {
-                    const PassDF r = long_pass<NW, 0>(G, m, w, Wf, W, E, k, sum, sh);
-                    ++n_pass;
-                    if (r.count > w.v) hi2 = fmin(hi2, E);
-                    else lo2 = fmax(lo2, E);
-                    const double En = E + r.dE;
-                    if (!isfinite(En) || !(En >= lo2 && En <= hi2) || r.nodes != w.v) break;
-                    // the FP32 sum of the group pass is accurate to ~1e-6 (chunk
-                    // sums of a few hundred terms), so one step from within 1e-8
-                    // leaves ~1e-14: the first pass settles
-                    done = fabs(r.dE) <= (it == 0 ? 1e-8 * fmax(1.0, fabs(E)) : 1e-12 * fmax(1.0, fabs(E)));
-                    E = En;
-                }
-                if (done) {
-                    lo = lo2;
-                    hi = hi2;
-                }
-            }
-        }
-        if (!done) {
-            // ---- stage 3: the FP32 bracket may be off by its count errors:
-            // restart from the scan bracket widened by one trial spacing
-            lo = fmax(m.e_lo, w.lo0 - m.delta);
-            hi = fmin(m.e_cap, w.hi0 + m.delta);
-            if (!(E > lo && E < hi)) E = 0.5 * (lo + hi);
-            bool moved_last = false;
-            for (int it = 0, cap = fallback_cap(b); it < cap; ++it) {
-                const PassDF r = long_pass<NW, 1>(G, m, w, Wf, W, E, k, 1.0, sh);
-                ++n_pass;
-                sum = r.sum;
-                if (r.count > w.v) hi = E;
-                else lo = E;
-                if (r.peak_log2 >= 2 && !moved_last) {
-                    k = clamp_k(w, r.peak_i);
-                    moved_last = true;
-                    continue;  // the same energy at the new match point
-                }
-                moved_last = false;
-                const double tol = 1e-12 * fmax(1.0, fabs(E));
-                const double En = E + r.dE;
-                const bool near = r.nodes == w.v || (m.status & EPSCU_STATUS_UNDER);
-                if (near && isfinite(En) && En > lo && En < hi) {
-                    E = En;
-                    if (fabs(r.dE) <= tol) {
-                        done = true;
-                        break;
-                    }
-                } else {
-                    E = 0.5 * (lo + hi);
-                }
-                if (hi - lo <= tol) {
-                    E = 0.5 * (lo + hi);
+            moved_last = false;
+            const double tol = 1e-12 * fmax(1.0, fabs(E));
+            const double En = E + r.dE;
+            const bool near = r.nodes == w.v || (m.status & EPSCU_STATUS_UNDER);
+            if (near && isfinite(En) && En > lo && En < hi) {
+                E = En;
+                if (fabs(r.dE) <= tol) {
                     done = true;
                     break;
                 }
+            } else {
+                E = 0.5 * (lo + hi);
+            }
+            if (hi - lo <= tol) {
+                E = 0.5 * (lo + hi);
+                done = true;
+                break;
             }
         }
-        if (G.leader()) {
-            if (!done) w.status |= EPSCU_STATUS_MAXITER;
-            w.lo = lo;
-            w.hi = hi;
-            w.E = E;
-            w.k = k;
-            w.norm_k_in = sum;
-            w.iters = n_pass32 + n_pass;
-            const unsigned long long pts = (unsigned long long)(w.j1 - w.j0);
-            atomicAdd(&b.hdr->refine_updates, (unsigned long long)n_pass32 * pts);
-            atomicAdd(&b.hdr->df_updates, (unsigned long long)n_pass * pts);
-            if (mode == 0 && NW == kLongWarps) {
-                atomicAdd(&b.hdr->long32_updates, (unsigned long long)n_pass32 * pts);
-                atomicAdd(&b.hdr->longdf_updates, (unsigned long long)n_pass * pts);
-            }
-            b.levels[slot] = w;
-        }
+    }
+    if (!done) w.status |= EPSCU_STATUS_MAXITER;
+    w.lo = lo;
+    w.hi = hi;
+    w.E = E;
+    w.k = k;
+    w.norm_k_in = sum;
+    w.iters = n_pass32 + n_pass;
+    if (G.leader()) {
+        const unsigned long long pts = (unsigned long long)(w.j1 - w.j0);
+        atomicAdd(&b.hdr->refine_updates, (unsigned long long)n_pass32 * pts);
+        atomicAdd(&b.hdr->df_updates, (unsigned long long)n_pass * pts);
     }
 }
 
-// The norm pass of a group level and its match-point candidates (as
-// norm_df).  With psi requested every pass also stores its unnormalised
-// psi-hat in the level's row (MODE 3) and the last pass is the one kept;
-// scale_psi applies the constants afterwards.
-template <int NW>
-__global__ void __launch_bounds__(kLongThreads, kLongCtasPerSm) norm_long_kernel(DevBatch b, const int32_t* list,
-                                                                 const int32_t* list_len, int qid) {
-    constexpr int kG = kLongThreads / (32 * NW);
-    __shared__ SharedDF<NW> shd[kG];
-    const Grp<NW> G;
-    SharedDF<NW>& sh = shd[G.g()];
-    const int n = min(*list_len, b.max_levels);
+// The norm pass of a level and its match-point candidates (as norm_df_level).
+// With psi requested every pass also stores its unnormalised psi-hat (MODE 3)
+// and the last pass is the one kept.  Returns whether the twist search is due.
+__device__ __noinline__ bool norm_cta(const Grp& G, const DevBatch& b, LevelWork& w, double* row, SharedDF& sh) {
+    const PotMeta m = b.meta[w.p];
+    const float2* Wf = b.Wf2 + m.offf;
+    const double* W = b.W64 + m.off;
+    auto pass = [&](int kk) { return long_pass<3>(G, m, w, Wf, W, w.E, kk, 1.0, sh, row); };
+    int k = w.k;
+    PassDF r = pass(k);
+    if (r.peak_log2 >= 2) {
+        k = clamp_k(w, r.peak_i);
+        r = pass(k);
+    }
+    int k_row = k;  // the pass whose psi-hat the row holds
+    if (r.nodes != w.v) {
+        const int kt = grp_bcast(G, G.leader() ? clamp_k(w, match_index(m, b.Msuf, w.E)) : 0, sh.word);
+        PassDF r2 = pass(kt);
+        int k2 = kt;
+        if (r2.nodes != w.v && r2.peak_log2 >= 1) {
+            k2 = clamp_k(w, r2.peak_i);
+            r2 = pass(k2);
+        }
+        k_row = k2;
+        if (r2.nodes == w.v) {
+            r = r2;
+            k = k2;
+        }
+    }
+    if (redo_norm(w, r)) {
+        if (G.leader()) atomicAdd(&b.hdr->n_redo, 1);
+        w.E += r.dE;
+        r = pass(k);
+    } else if (row && k_row != k) {
+        r = pass(k);
+    }
+    finalize_df(m, w, r, k);
+    return suspicious(m, w, r.nodes, r.dE);
+}
+
+// Twist-index search for a flagged level (any window length): a chunked
+// outward sweep stores D/A every kTwistSample points, a chunked inward sweep
+// forms |gamma_k| at the same points, the match point becomes argmin
+// |gamma_k| (Dhillon and Parlett's twisted-factorisation rule), then Newton
+// and the norm pass run there.
+__device__ __noinline__ void twist_cta(const Grp& G, const DevBatch& b, LevelWork& w, double* row, SharedDF& sh) {
+    const PotMeta m = b.meta[w.p];
+    const float2* Wf = b.Wf2 + m.offf;
+    const double* W = b.W64 + m.off;
+    const dfl aE = energy_df(m, w.E);
+    TwistIO tw;
+    tw.rho = b.twist_scratch + (int64_t)(kFragileScratch + blockIdx.x) * b.twist_stride;
+    tw.W = W;
+    tw.aEd = __dmul_rn(m.a, w.E);
+    tw.j0 = w.j0;
+    tw.j1 = w.j1;
+    tw.stride = b.twist_stride;
+    tw.best = INFINITY;
+    tw.k = w.k;
+    long_side<4>(G, Wf, aE, w.j0, w.j1, +1, nullptr, 0.0, 0, sh, &tw);
+    long_side<5>(G, Wf, aE, w.j1, w.j0, -1, nullptr, 0.0, 0, sh, &tw);
+    const int k = clamp_k(w, tw.k == 0x7fffffff ? w.k : tw.k);
+    auto pass = [&](double e) { return long_pass<3>(G, m, w, Wf, W, e, k, 1.0, sh, row); };
+    double E1 = w.E;
+    PassDF r = pass(E1);
+    for (int it = 0; it < 8; ++it) {
+        if (r.nodes != w.v || !isfinite(r.dE) || !(fabs(r.dE) < 1e-7)) break;
+        if (fabs(r.dE) <= 1e-13 * fmax(1.0, fabs(E1))) break;
+        E1 += r.dE;
+        r = pass(E1);
+    }
+    w.E = E1;
+    finalize_df(m, w, r, k);
+}
+
+// ---------------------------------------------------------------- kernels
+
+// levels to a warp, two lanes each (the windows and pass counts differ, and the
+// levels are few: more to a warp would only lengthen it)
+constexpr int kLaneLevels = 8;
+
+__device__ __forceinline__ bool next_levels(const DevBatch& b, int qid, int per, int2& unit) {
+    int u = 0;
+    if ((threadIdx.x & 31) == 0) u = atomicAdd(&b.hdr->queue[qid], 1);
+    u = __shfl_sync(0xffffffffu, u, 0);
+    const int n = min(b.hdr->n_fragile, b.max_levels);
+    if (u >= (n + per - 1) / per) return false;
+    unit = make_int2(u * per, min(per, n - u * per));
+    return true;
+}
+
+// The fragile levels: the CTAs first take the long windows, a CTA each, then
+// their warps the others, of similar window length and longest first: FP32
+// refinement, double-float Newton and norm pass back to back, then the rows by
+// the warp.
+__global__ void __launch_bounds__(kLongThreads, kLongCtasPerSm) fragile_kernel(DevBatch b) {
+    __shared__ SharedDF sh;
+    __shared__ Shared32 sh32;
+    const Grp G;
+    const int n_long = min(b.hdr->n_fragile_long, b.max_levels);
     for (;;) {
-        const int q = grp_next<NW>(G, &b.hdr->queue[qid], sh.word);
-        if (q >= n) break;
-        const int slot = list[q];
+        const int q = grp_next(G, &b.hdr->queue[kQFragileLong], sh.word);
+        if (q >= n_long) break;
+        const int slot = b.fragile_long[q];
         LevelWork w = b.levels[slot];
-        if (w.status & (EPSCU_STATUS_NOTFOUND | EPSCU_STATUS_CANCELLED)) continue;
-        const PotMeta m = b.meta[w.p];
-        const float2* Wf = b.Wf2 + m.offf;
-        const double* W = b.W64 + m.off;
-        double* row = psi_row(b, m, w);
-        auto pass = [&](int kk) { return long_pass<NW, 3>(G, m, w, Wf, W, w.E, kk, 1.0, sh, row); };
-        int k = w.k;
-        PassDF r = pass(k);
-        if (r.peak_log2 >= 2) {
-            k = clamp_k(w, r.peak_i);
-            r = pass(k);
+        double* row = psi_row(b, b.meta[w.p], w);
+        bool off = false;
+        if (grp_cancelled(G, b, sh.word)) {
+            w.status |= EPSCU_STATUS_CANCELLED;
+        } else {
+            refine_cta(G, b, w, false, sh, sh32);
+            off = norm_cta(G, b, w, row, sh);
         }
-        int k_row = k;  // the pass whose psi-hat the row holds
-        if (r.nodes != w.v) {
-            const int kt = grp_bcast<NW>(G, G.leader() ? clamp_k(w, match_index(m, b.Msuf, w.E)) : 0, sh.word);
-            PassDF r2 = pass(kt);
-            int k2 = kt;
-            if (r2.nodes != w.v && r2.peak_log2 >= 1) {
-                k2 = clamp_k(w, r2.peak_i);
-                r2 = pass(k2);
-            }
-            k_row = k2;
-            if (r2.nodes == w.v) {
-                r = r2;
-                k = k2;
-            }
-        }
-        if (redo_norm(w, r)) {
-            if (G.leader()) atomicAdd(&b.hdr->n_redo, 1);
-            w.E += r.dE;
-            r = pass(k);
-        } else if (row && k_row != k) {
-            r = pass(k);
-        }
+        if (row) finish_row<kLongThreads>(G.t(), w, row, b.meta[w.p].N);
         if (G.leader()) {
-            finalize_df(m, w, r, k);
-            if (suspicious(m, w, r.nodes, r.dE) && b.twist_list) {
-                const int t = atomicAdd(&b.hdr->n_twist, 1);
-                if (t < b.max_twist) b.twist_list[t] = slot;
-            }
             b.levels[slot] = w;
+            if (off && b.fragile_twist) {
+                const int t = atomicAdd(&b.hdr->n_fragile_twist, 1);
+                if (t < b.max_twist) b.fragile_twist[t] = slot;
+            }
+        }
+    }
+    const int lane = threadIdx.x & 31;
+    for (int2 unit; next_levels(b, kQFragileLanes, kLaneLevels, unit);) {
+        if (lane / 2 < unit.y) {
+            const int slot = b.fragile_list[unit.x + lane / 2];
+            refine32_level(b, slot);
+            newton_df_level(b, slot);
+            norm_df_level(b, slot);
+        }
+        __syncwarp();
+        if (!b.psi || b.hdr->error) continue;
+        for (int u = 0; u < unit.y; ++u) {
+            const LevelWork w = b.levels[b.fragile_list[unit.x + u]];
+            if (w.status & EPSCU_STATUS_FALLBACK) continue;
+            const PotMeta& m = b.meta[w.p];
+            finish_row<32>(lane, w, psi_row(b, m, w), m.N);
         }
     }
 }
 
-// Twist-index search for the levels the norm passes flagged (any window
-// length): a chunked outward sweep stores D/A every kTwistSample points, a
-// chunked inward sweep forms |gamma_k| at the same points, the match point
-// becomes argmin |gamma_k| (Dhillon and Parlett's twisted-factorisation
-// rule), then Newton and the norm pass run there; with psi requested the
-// final pass stores the unnormalised psi-hat in the level's row (scale_psi
-// applies the constants).  The level joins the long list, so the adjoint's
-// recompute path (write_long) writes its psi.  One CTA per level.
-__global__ void __launch_bounds__(kLongThreads, kLongCtasPerSm) twist_long_kernel(DevBatch b) {
-    __shared__ SharedDF<kLongWarps> sh;
-    const Grp<kLongWarps> G;
-    const int n = min(b.hdr->n_twist, b.max_twist);
+// Levels the lane Newton handed over (refinement from the scan bracket
+// widened by one trial spacing, norm pass), then those whose final pass
+// disagrees.  Theirs are the CTA passes' constants from here on.
+__global__ void __launch_bounds__(kLongThreads, kLongCtasPerSm) fragile_repair_kernel(DevBatch b) {
+    __shared__ SharedDF sh;
+    __shared__ Shared32 sh32;
+    const Grp G;
+    const int n_fall = min(b.hdr->n_fragile_fall, b.max_levels);
+    const int n_twist = min(b.hdr->n_fragile_twist, b.max_twist);
     for (;;) {
-        const int q = grp_next<kLongWarps>(G, &b.hdr->queue[kQTwistLong], sh.word);
-        if (q >= n) break;
-        const int slot = b.twist_list[q];
+        const int q = grp_next(G, &b.hdr->queue[kQFragileRepair], sh.word);
+        if (q >= n_fall + n_twist) break;
+        const int slot = q < n_fall ? b.fragile_fall[q] : b.fragile_twist[q - n_fall];
         LevelWork w = b.levels[slot];
-        const PotMeta m = b.meta[w.p];
-        const float2* Wf = b.Wf2 + m.offf;
-        const double* W = b.W64 + m.off;
-        const dfl aE = energy_df(m, w.E);
-        TwistIO tw;
-        tw.rho = b.twist_scratch + (int64_t)q * b.twist_stride;
-        tw.W = W;
-        tw.aEd = __dmul_rn(m.a, w.E);
-        tw.j0 = w.j0;
-        tw.j1 = w.j1;
-        tw.stride = b.twist_stride;
-        tw.best = INFINITY;
-        tw.k = w.k;
-        long_side<kLongWarps, 4>(G, Wf, aE, w.j0, w.j1, +1, nullptr, 0.0, 0, sh, &tw);
-        long_side<kLongWarps, 5>(G, Wf, aE, w.j1, w.j0, -1, nullptr, 0.0, 0, sh, &tw);
-        const int k = clamp_k(w, tw.k == 0x7fffffff ? w.k : tw.k);
-        double* row = psi_row(b, m, w);
-        auto pass = [&](double e) { return long_pass<kLongWarps, 3>(G, m, w, Wf, W, e, k, 1.0, sh, row); };
-        double E1 = w.E;
-        PassDF r = pass(E1);
-        for (int it = 0; it < 8; ++it) {
-            if (r.nodes != w.v || !isfinite(r.dE) || !(fabs(r.dE) < 1e-7)) break;
-            if (fabs(r.dE) <= 1e-13 * fmax(1.0, fabs(E1))) break;
-            E1 += r.dE;
-            r = pass(E1);
+        double* row = psi_row(b, b.meta[w.p], w);
+        bool off = true;
+        if (q < n_fall) {
+            if (grp_cancelled(G, b, sh.word)) {
+                w.status |= EPSCU_STATUS_CANCELLED;
+                off = false;
+            } else {
+                refine_cta(G, b, w, true, sh, sh32);
+                off = norm_cta(G, b, w, row, sh) && b.fragile_twist;
+            }
         }
-        w.E = E1;
+        if (off) twist_cta(G, b, w, row, sh);
+        if (row) finish_row<kLongThreads>(G.t(), w, row, b.meta[w.p].N);
         if (G.leader()) {
-            finalize_df(m, w, r, k);
-            if (!(w.status & EPSCU_STATUS_LONG) && b.long_list) {
-                const int t = atomicAdd(&b.hdr->n_long, 1);
-                if (t < b.max_levels) {
-                    b.long_list[t] = slot;
-                    w.status |= EPSCU_STATUS_LONG;
-                }
+            if (!is_long(w) && !(w.status & EPSCU_STATUS_FALLBACK)) {
+                const int t = atomicAdd(&b.hdr->n_fragile_long, 1);
+                if (t < b.max_levels) b.fragile_long[t] = slot;
+                w.status |= EPSCU_STATUS_LONG;
             }
             b.levels[slot] = w;
         }
     }
 }
 
-// psi of the listed levels in FP64 from the final constants (window points
-// and psi_k; the rest of each row is zero): the adjoint's recompute path.
-// One CTA per level.
-__global__ void __launch_bounds__(kLongThreads, kLongCtasPerSm) write_long_kernel(DevBatch b, const int32_t* list,
-                                                                  const int32_t* list_len) {
-    __shared__ SharedDF<kLongWarps> sh;
-    const Grp<kLongWarps> G;
+// psi again from the final constants (the adjoint of a solve that kept none):
+// the rows' zeros (the whole row of a level without a result), then the
+// windows, a lane per level and a CTA for the long and the handed-over levels.
+__global__ void __launch_bounds__(256) fragile_zero_kernel(DevBatch b) {
     if (!b.psi || b.hdr->error) return;
-    const int n = min(*list_len, b.max_levels);
-    for (int q = blockIdx.x; q < n; q += gridDim.x) {
-        const int slot = list[q];
+    const int lane = threadIdx.x & 31;
+    const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, n_warps = (gridDim.x * blockDim.x) >> 5;
+    const int total = b.hdr->total_levels;
+    for (int slot = warp; slot < total; slot += n_warps) {
         const LevelWork w = b.levels[slot];
+        if (w.bucket < kListFragile * kBuckets) continue;
+        const int N = b.meta[w.p].N;
+        double* row = psi_row(b, b.meta[w.p], w);
+        const bool none = no_result(w);
+        zero_points<32>(lane, row, none ? N : w.j0);
+        if (!none) zero_points<32>(lane, row + w.j1 + 1, N - 1 - w.j1);
+    }
+}
+
+__global__ void __launch_bounds__(128) fragile_write_lanes_kernel(DevBatch b) {
+    if (!b.psi || b.hdr->error) return;
+    const int lane = threadIdx.x & 31;
+    for (int2 unit; next_levels(b, kQFragileRewrite, 32, unit);) {
+        if (lane >= unit.y) continue;
+        const LevelWork w = b.levels[b.fragile_list[unit.x + lane]];
+        if (no_result(w) || is_long(w) || (w.status & EPSCU_STATUS_FALLBACK)) continue;
         const PotMeta m = b.meta[w.p];
-        double* out = b.psi + m.psi_off + (int64_t)(w.v - b.min_level) * m.N;
-        // the rows were zeroed by zero_psi: only the window is written
-        if (no_result(w)) continue;
+        double* out = psi_row(b, m, w);
         const float2* Wf = b.Wf2 + m.offf;
         const dfl aE = energy_df(m, w.E);
-        long_side<kLongWarps, 2>(G, Wf, aE, w.j0, w.k, +1, out, w.norm_k_out, w.ex_out, sh);
-        long_side<kLongWarps, 2>(G, Wf, aE, w.j1, w.k, -1, out, w.norm_k_in, w.ex_in, sh);
-        if (threadIdx.x == 0) out[w.k] = w.ck;
+        SideDF<2> st;
+        side_df<2>(Wf, aE, w.j0, w.k, +1, st, out, w.norm_k_out, w.ex_out);
+        side_df<2>(Wf, aE, w.j1, w.k, -1, st, out, w.norm_k_in, w.ex_in);
+        out[w.k] = w.ck;
+    }
+}
+
+__global__ void __launch_bounds__(kLongThreads, kLongCtasPerSm) fragile_write_long_kernel(DevBatch b) {
+    __shared__ SharedDF sh;
+    const Grp G;
+    if (!b.psi || b.hdr->error) return;
+    const int n_long = min(b.hdr->n_fragile_long, b.max_levels), n_fall = min(b.hdr->n_fragile_fall, b.max_levels);
+    for (int q = blockIdx.x; q < n_long + n_fall; q += gridDim.x) {
+        const LevelWork w = b.levels[q < n_long ? b.fragile_long[q] : b.fragile_fall[q - n_long]];
+        if (no_result(w)) continue;
+        const PotMeta m = b.meta[w.p];
+        double* out = psi_row(b, m, w);
+        const float2* Wf = b.Wf2 + m.offf;
+        const dfl aE = energy_df(m, w.E);
+        long_side<2>(G, Wf, aE, w.j0, w.k, +1, out, w.norm_k_out, w.ex_out, sh);
+        long_side<2>(G, Wf, aE, w.j1, w.k, -1, out, w.norm_k_in, w.ex_in, sh);
+        if (G.leader()) out[w.k] = w.ck;
         __syncthreads();  // the shared scratch is reused by the next level
     }
 }
 
 }  // namespace
 
-void launch_refine_long(const DevBatch& b, int sm_count, cudaStream_t s) {
-    if (!b.long_list) return;
-    refine_long_kernel<kLongWarps>
-        <<<sm_count * kLongCtasPerSm, kLongThreads, 0, s>>>(b, 0, b.long_list, &b.hdr->n_long, kQLongRefine);
+void launch_fragile(const DevBatch& b, int sm_count, cudaStream_t s) {
+    fragile_kernel<<<sm_count * kLongCtasPerSm, kLongThreads, 0, s>>>(b);
 }
-void launch_fallback_long(const DevBatch& b, int sm_count, cudaStream_t s) {
-    if (!b.fallback_list) return;
-    refine_long_kernel<kLongWarps>
-        <<<sm_count * kLongCtasPerSm, kLongThreads, 0, s>>>(b, 1, b.fallback_list, &b.hdr->fallbacks, kQFallback);
+void launch_fragile_repair(const DevBatch& b, int sm_count, cudaStream_t s) {
+    fragile_repair_kernel<<<sm_count * kLongCtasPerSm, kLongThreads, 0, s>>>(b);
 }
-void launch_norm_long(const DevBatch& b, int sm_count, cudaStream_t s) {
-    if (!b.long_list) return;
-    norm_long_kernel<kLongWarps><<<sm_count * kLongCtasPerSm, kLongThreads, 0, s>>>(b, b.long_list, &b.hdr->n_long, kQNormLong);
-}
-void launch_norm_fallback(const DevBatch& b, int sm_count, cudaStream_t s) {
-    if (!b.fallback_list) return;
-    norm_long_kernel<kLongWarps>
-        <<<sm_count * kLongCtasPerSm, kLongThreads, 0, s>>>(b, b.fallback_list, &b.hdr->fallbacks, kQNormFallback);
-}
-void launch_twist_long(const DevBatch& b, int sm_count, cudaStream_t s) {
-    if (!b.twist_list || !b.long_list) return;
-    twist_long_kernel<<<sm_count * kLongCtasPerSm, kLongThreads, 0, s>>>(b);
-}
-void launch_write_long(const DevBatch& b, int sm_count, cudaStream_t s) {
-    // the group levels of both tiers (the recompute path: one CTA per level)
-    if (b.long_list) write_long_kernel<<<sm_count * kLongCtasPerSm, kLongThreads, 0, s>>>(b, b.long_list, &b.hdr->n_long);
-    if (b.mid_list) write_long_kernel<<<sm_count * kLongCtasPerSm, kLongThreads, 0, s>>>(b, b.mid_list, &b.hdr->n_mid);
-    if (b.fallback_list)
-        write_long_kernel<<<sm_count * kLongCtasPerSm, kLongThreads, 0, s>>>(b, b.fallback_list, &b.hdr->fallbacks);
-}
-// the middle tier is in use (its list can be non-empty): the same threshold
-// as the window kernel's
-static bool mid_tier_on(const DevBatch& b) {
-    return b.mid_list && (b.mid_window != 0 ? b.mid_window : kMidWindow) > 0;
-}
-void launch_refine_mid(const DevBatch& b, int sm_count, cudaStream_t s) {
-    if (!mid_tier_on(b)) return;
-    refine_long_kernel<1><<<sm_count * kLongCtasPerSm, kLongThreads, 0, s>>>(b, 2, b.mid_list, &b.hdr->n_mid, kQMidRefine);
-}
-void launch_norm_mid(const DevBatch& b, int sm_count, cudaStream_t s) {
-    if (!mid_tier_on(b)) return;
-    norm_long_kernel<1><<<sm_count * kLongCtasPerSm, kLongThreads, 0, s>>>(b, b.mid_list, &b.hdr->n_mid, kQNormMid);
+void launch_fragile_rewrite(const DevBatch& b, int sm_count, cudaStream_t s) {
+    fragile_zero_kernel<<<sm_count * 8, 256, 0, s>>>(b);
+    fragile_write_lanes_kernel<<<sm_count * 8, 128, 0, s>>>(b);
+    fragile_write_long_kernel<<<sm_count * kLongCtasPerSm, kLongThreads, 0, s>>>(b);
 }
 
 }  // namespace epscu

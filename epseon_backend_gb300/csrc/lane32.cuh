@@ -1,6 +1,5 @@
-// lane32.cuh -- the FP32 lane pass of the fast method and the per-level
-// refinement built on it (one lane per level), shared by refine32_kernel
-// (levels.cu) and the fused lane kernel (polish.cu).
+// lane32.cuh -- the FP32 lane pass and the per-level refinement built on it,
+// two lanes per level (fragile.cu).
 #pragma once
 
 #include <math.h>
@@ -92,37 +91,31 @@ __device__ __forceinline__ void side32_rest(Side32& s, const float2* __restrict_
     }
 }
 
+// The two lanes of a pair (2 l, 2 l + 1) work on one level, the even one
+// marching the outward side of every pass, the odd one the inward side (two
+// independent recurrences), and hand each other the result: a pass lasts as
+// long as its longer side, the operations are those of one lane doing both.
+// Everything else both lanes do alike.
+__device__ __forceinline__ unsigned pair_mask() { return 3u << (threadIdx.x & 30); }
+__device__ __forceinline__ bool inward_lane() { return (threadIdx.x & 1) != 0; }
+__device__ __forceinline__ int pair_other(int v) { return __shfl_xor_sync(pair_mask(), v, 1); }
+__device__ __forceinline__ float pair_other(float v) { return __shfl_xor_sync(pair_mask(), v, 1); }
+__device__ __forceinline__ double pair_other(double v) { return __shfl_xor_sync(pair_mask(), v, 1); }
+// the even lane's value
+__device__ __forceinline__ int pair_first(int v) { return __shfl_sync(pair_mask(), v, threadIdx.x & 30); }
+
 __device__ __forceinline__ Pass32 cooley32(const PotMeta& m, const float2* __restrict__ Wf, const double* __restrict__ W64,
                                            double E, int k, int j0, int j1) {
     const double aE = __dmul_rn(m.a, E);
     const float aEh = __double2float_rn(aE);
     const float aEl = __double2float_rn(aE - (double)aEh);
     // outward from j0 (u_{j0} = 1, u_{j0-1} = 0) and inward from j1, both to k
-    Side32 o{1.0f, 1.0f, 0.0f, 0, 0, -(1 << 30), j0};
-    Side32 in{1.0f, 1.0f, 0.0f, 0, 0, -(1 << 30), j1};
-    const int no = k - j0, ni = j1 - k;
-    // the two sides are independent recurrences: their common full chunks run
-    // interleaved (two dependency chains per lane), the rest of the longer
-    // side alone; the arithmetic of each side is unchanged
-    const int nb = min(no, ni) & ~7;
-    int base = 0;
-    for (; base < nb; base += 8) {
-        float2 wo[8], wi[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            wo[u] = __ldg(Wf + j0 + base + u);
-            wi[u] = __ldg(Wf + j1 - base - u);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            step32s(o, aEh, aEl, wo[u]);
-            step32s(in, aEh, aEl, wi[u]);
-        }
-        renorm32s(o, j0 + base + 7);
-        renorm32s(in, j1 - base - 7);
-    }
-    side32_rest(o, Wf, aEh, aEl, j0, +1, base, no);
-    side32_rest(in, Wf, aEh, aEl, j1, -1, base, ni);
+    const bool inw = inward_lane();
+    Side32 mine{1.0f, 1.0f, 0.0f, 0, 0, -(1 << 30), inw ? j1 : j0};
+    side32_rest(mine, Wf, aEh, aEl, inw ? j1 : j0, inw ? -1 : 1, 0, inw ? j1 - k : k - j0);
+    const Side32 other{pair_other(mine.A),    pair_other(mine.D),   pair_other(mine.S), pair_other(mine.ecum),
+                       pair_other(mine.nodes), pair_other(mine.Lpk), pair_other(mine.ipk)};
+    const Side32 o = inw ? other : mine, in = inw ? mine : other;
     const int nodes = o.nodes + in.nodes;
     const float Ao = o.A, Do = o.D, So = o.S, Ai = in.A, Di = in.D, Si = in.S;
     const int Lk[2] = {o.ecum + (o.A != 0.0f ? ((__float_as_int(fabsf(o.A)) >> 23) & 0xff) : -1000),
@@ -161,13 +154,13 @@ constexpr double kTol32 = 2e-9;
 // redo, +0.6 and +2.6 ms a step.)
 constexpr double kAccept32 = 2e-9;
 
-// The FP32 refinement of the level in slot `slot` (one lane); false when the
+// The FP32 refinement of the level in slot `slot` (a lane pair); false when the
 // level takes no lane refinement (no bracket, a long window, or cancelled).
 __device__ __forceinline__ bool refine32_level(const DevBatch& b, int slot) {
     LevelWork w = b.levels[slot];
-    // long windows: refine_long (middle windows take their FP32 passes here)
+    // (long windows take the CTA passes)
     if (w.status & (EPSCU_STATUS_NOTFOUND | EPSCU_STATUS_LONG)) return false;
-    if (cancelled(b)) {
+    if (pair_first(cancelled(b))) {
         b.levels[slot].status = w.status | EPSCU_STATUS_CANCELLED;
         return false;
     }
@@ -245,9 +238,12 @@ __device__ __forceinline__ bool refine32_level(const DevBatch& b, int slot) {
     w.norm_k_in = sum;  // sum psi~^2 at the match point k, the Newton denominator of newton_df
     w.iters = it;
     const unsigned long long upd = (unsigned long long)(it + 1) * (unsigned long long)(w.j1 - w.j0);
-    atomicAdd(&b.hdr->refine_updates, upd);
-    atomicMax(&b.hdr->refine_max_updates, upd);
-    atomicMax(&b.hdr->refine_max_iters, it + 1);
+    if (!inward_lane()) {
+        atomicAdd(&b.hdr->refine_updates, upd);
+        atomicMax(&b.hdr->refine_max_updates, upd);
+        atomicMax(&b.hdr->refine_max_iters, it + 1);
+    }
+    __syncwarp(pair_mask());
     b.levels[slot] = w;
     return true;
 }

@@ -1,6 +1,5 @@
-// lanedf.cuh -- the double-float lane passes of the fast method (one lane
-// per level) and the per-level Newton and norm stages built on them, shared
-// by newton_df_kernel / norm_df_kernel and the fused lane kernel (polish.cu).
+// lanedf.cuh -- the double-float lane passes (two lanes per level) and the
+// per-level Newton and norm stages built on them (fragile.cu).
 //
 // The recurrence of the last passes runs in double-float arithmetic (~48-bit
 // significands, see dfloat.cuh) in the Blatt difference form
@@ -144,47 +143,33 @@ __device__ __forceinline__ void side_df(const float2* __restrict__ Wf, dfl aE, i
     if (MODE == 1 || MODE == 3) st.S = st.ss.value();
 }
 
-// one pass at E with match point k over the level's window [w.j0, w.j1];
-// MODE 0: gamma/count only, MODE 1: + sums, MODE 3: + unnormalised psi-hat
-// into row (the level's psi row).  PAIRED: the outward and inward sides are
-// independent recurrences, so their common full chunks can run interleaved
-// (two dependency chains per lane) and the rest of the longer side alone; the
-// arithmetic of each side is unchanged.  (Measured on GB300: slower for both
-// the state-only Newton pass and the norm pass, whose doubled loop bodies
-// cost more than the second chain gains; the FP32 lane pass, with a far
-// shorter step, does gain from it.)
-template <int MODE, bool PAIRED>
+// one pass at E with match point k over the level's window [w.j0, w.j1], a
+// side on each lane of the pair; MODE 0: gamma/count only, MODE 1: + sums,
+// MODE 3: + unnormalised psi-hat into row (the level's psi row)
+template <int MODE>
 __device__ PassDF pass_df(const PotMeta& m, const LevelWork& w, const float2* __restrict__ Wf,
                           const double* __restrict__ W64, double E, int k, double sum_fallback,
                           double* __restrict__ row = nullptr) {
     const dfl aE = energy_df(m, E);
-    SideDF<MODE> o, in;
-    o.init(w.j0, 0.0, 0);
-    in.init(w.j1, 0.0, 0);
-    const int no = k - w.j0, ni = w.j1 - k;
-    const int nb = PAIRED ? (min(no, ni) & ~7) : 0;
-    int base = 0;
-    for (; base < nb; base += 8) {
-        float2 wo[8], wi[8];
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            wo[u] = __ldg(Wf + w.j0 + base + u);
-            wi[u] = __ldg(Wf + w.j1 - base - u);
-        }
-#pragma unroll
-        for (int u = 0; u < 8; ++u) {
-            o.step(aE, wo[u], row, w.j0 + base + u);
-            in.step(aE, wi[u], row, w.j1 - base - u);
-        }
-        o.renorm(w.j0 + base + 7);
-        in.renorm(w.j1 - base - 7);
-    }
-    side_df_rest(o, Wf, aE, w.j0, +1, base, no, row);
-    side_df_rest(in, Wf, aE, w.j1, -1, base, ni, row);
+    const bool inw = inward_lane();
+    SideDF<MODE> mine;
+    mine.init(inw ? w.j1 : w.j0, 0.0, 0);
+    side_df_rest(mine, Wf, aE, inw ? w.j1 : w.j0, inw ? -1 : 1, 0, inw ? w.j1 - k : k - w.j0, row);
+    if (MODE == 1 || MODE == 3) mine.S = mine.ss.value();
+    SideDF<MODE> other;
+    other.A = {pair_other(mine.A.h), pair_other(mine.A.l)};
+    other.D = {pair_other(mine.D.h), pair_other(mine.D.l)};
+    other.nodes = pair_other(mine.nodes);
     if (MODE == 1 || MODE == 3) {
-        o.S = o.ss.value();
-        in.S = in.ss.value();
+        other.q = {pair_other(mine.q.h), pair_other(mine.q.l)};
+        other.eA = pair_other(mine.eA);
+        other.eQ = pair_other(mine.eQ);
+        other.S = pair_other(mine.S);
+        other.peak_L = pair_other(mine.peak_L);
+        other.peak_i = pair_other(mine.peak_i);
     }
+    const SideDF<MODE>& o = inw ? other : mine;
+    const SideDF<MODE>& in = inw ? mine : other;
     const double Tk = __dsub_rn(__dmul_rn(m.a, E), __ldg(W64 + k));
     const double fk = 1.0 + Tk;
     const double Ao = df_to_double(o.A), Do = df_to_double(o.D);
@@ -233,7 +218,7 @@ __device__ __forceinline__ bool newton_df_level(const DevBatch& b, int slot) {
     bool ok = false;
     int n_pass = 0;
     for (int it = 0; it < 4 && !ok; ++it) {
-        const PassDF r = pass_df<0, false>(m, w, Wf, W, E, w.k, w.norm_k_in);
+        const PassDF r = pass_df<0>(m, w, Wf, W, E, w.k, w.norm_k_in);
         ++n_pass;
         if (r.count > w.v) hi = fmin(hi, E);
         else lo = fmax(lo, E);
@@ -250,16 +235,19 @@ __device__ __forceinline__ bool newton_df_level(const DevBatch& b, int slot) {
         // hand the level to the bisection fallback kernel (so this warp
         // does not stall on it)
         w.status |= EPSCU_STATUS_FALLBACK;
-        const int q = atomicAdd(&b.hdr->fallbacks, 1);
-        if (q < b.max_levels) b.fallback_list[q] = slot;
+        if (!inward_lane()) {
+            const int q = atomicAdd(&b.hdr->n_fragile_fall, 1);
+            if (q < b.max_levels) b.fragile_fall[q] = slot;
+        }
     } else {
         w.E = E;
     }
-    {
+    if (!inward_lane()) {
         const unsigned long long upd = (unsigned long long)n_pass * (unsigned long long)(w.j1 - w.j0);
         atomicAdd(&b.hdr->df_updates, upd);
         atomicMax(&b.hdr->df_max_updates, upd);
     }
+    __syncwarp(pair_mask());
     b.levels[slot] = w;
     return ok;
 }
@@ -282,7 +270,7 @@ __device__ __forceinline__ bool norm_df_level(const DevBatch& b, int slot) {
     int n_pass = 0;
     auto pass = [&](int kk) {
         ++n_pass;
-        return row ? pass_df<3, false>(m, w, Wf, W, w.E, kk, 1.0, row) : pass_df<1, false>(m, w, Wf, W, w.E, kk, 1.0);
+        return row ? pass_df<3>(m, w, Wf, W, w.E, kk, 1.0, row) : pass_df<1>(m, w, Wf, W, w.E, kk, 1.0);
     };
     // match point candidates: the FP32 one, the peak of |psi| seen by this
     // pass, the outer turning point and its peak; the first whose
@@ -309,22 +297,23 @@ __device__ __forceinline__ bool norm_df_level(const DevBatch& b, int slot) {
         }
     }
     if (redo_norm(w, r)) {
-        atomicAdd(&b.hdr->n_redo, 1);
+        if (!inward_lane()) atomicAdd(&b.hdr->n_redo, 1);
         w.E += r.dE;
         r = pass(k);
     } else if (row && k_row != k) {
         r = pass(k);
     }
     finalize_df(m, w, r, k);
-    {
+    if (!inward_lane()) {
         const unsigned long long upd = (unsigned long long)n_pass * (unsigned long long)(w.j1 - w.j0);
         atomicAdd(&b.hdr->df_updates, upd);
         atomicMax(&b.hdr->df_max_updates, upd);
     }
-    if (suspicious(m, w, r.nodes, r.dE) && b.twist_list) {
-        const int q = atomicAdd(&b.hdr->n_twist, 1);
-        if (q < b.max_twist) b.twist_list[q] = slot;
+    if (suspicious(m, w, r.nodes, r.dE) && b.fragile_twist && !inward_lane()) {
+        const int q = atomicAdd(&b.hdr->n_fragile_twist, 1);
+        if (q < b.max_twist) b.fragile_twist[q] = slot;
     }
+    __syncwarp(pair_mask());
     b.levels[slot] = w;
     return true;
 }

@@ -24,7 +24,7 @@ struct DevBatch {
     float* gam;                // [n * n_trial] the scan's matching function f_k gamma_k at the counted trial
                                // energies (fast method: the refinement's first energy), or nullptr
     LevelWork* levels;         // [max_levels]
-    int32_t* fallback_list;    // [max_levels] slots handed to the bisection fallback
+    int32_t* fallback_list;    // [max_levels] slots handed to the repair kernel
     int2* units;               // [max_units] (first slot, count) per warp work unit
     int32_t max_units;
     int32_t* twist_list;       // [max_twist] slots for the twist-index search
@@ -36,7 +36,11 @@ struct DevBatch {
     int32_t* order;            // [n] potentials by decreasing cost
     int2* scan_win;            // [n * ceil(n_trial / kScanWinBlock)] scan windows, or nullptr (full grid)
     int32_t* long_list;        // [max_levels] slots with long windows (CTA-per-level passes), or nullptr
-    int32_t* mid_list;         // [max_levels] slots with middle windows (warp-per-level passes), or nullptr
+    int32_t* fragile_list;     // [max_levels] fragile levels (fragile.cu): a lane each, or nullptr
+    int32_t* fragile_long;     // [max_levels]   long windows, a CTA each
+    int32_t* fragile_fall;     // [max_levels]   handed over by the lane Newton
+    int32_t* fragile_twist;    // [max_twist]    for the twist-index search
+    int32_t* warp_list;        // [max_levels] the other slots (warp-per-level passes), or nullptr
     int32_t* bis_list;         // [n * n_trial] trial indices of the bisection scan's current round, or
                                // nullptr (every trial energy scanned)
     int32_t* bis_n;            // [n] entries of bis_list per potential
@@ -49,30 +53,20 @@ struct DevBatch {
     int32_t min_level, max_level;
     int32_t max_N;             // longest grid of the batch
     int32_t long_window;       // window length above which a level takes the CTA passes
-    int32_t mid_window;        // window length above which a level takes the warp passes (< 0: none)
     int32_t wait_polls;        // polls of a bounded wait on a staged scan tile (0: kWaitPolls)
     int32_t max_iter;          // cap on FP32 refinement passes (0: 48; fallback passes: twice it)
     double tol;
 };
 
 constexpr int kWaitPolls = 1 << 22;       // default bound of the TMA scan's mbarrier waits
-// persistent grid of the lane-per-level kernels (refine32, newton_df,
-// norm_df): threads per CTA and CTAs per SM launched (together 512 threads at
-// up to 128 registers, the whole register file)
-constexpr int kLaneThreads = 128;
-constexpr int kLaneCtasPerSm = 4;
 constexpr int kRefineMaxIter = 48;        // default cap on a level's FP32 refinement passes
 __device__ __forceinline__ int refine_cap(const DevBatch& b) { return b.max_iter > 0 ? b.max_iter : kRefineMaxIter; }
 // double-float fallback passes (bisection from the widened scan bracket)
 __device__ __forceinline__ int fallback_cap(const DevBatch& b) { return 2 * refine_cap(b); }
 
-// Warp-level work queue of the per-level kernels: units of up to 32
+// Warp-level work queue of the plain method's per-level kernels: units of up to 32
 // consecutive level slots of one potential, longest grids first.  Lane 0
 // takes the next unit and broadcasts it; false when the queue is drained.
-// (Measured slower on the mixed batch: units of levels sorted by window
-// length across potentials, and a lane-level state machine that hands each
-// lane a new level as soon as it finishes -- its divergent bookkeeping costs
-// more than the idle lanes it saves.)
 __device__ __forceinline__ bool next_unit(const DevBatch& b, int qid, int2& unit) {
     int u = 0;
     if ((threadIdx.x & 31) == 0) u = atomicAdd(&b.hdr->queue[qid], 1);
@@ -112,29 +106,25 @@ void scan32_set_attributes();
 
 // levels.cu
 void launch_bisect64(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_refine32(const DevBatch& b, int sm_count, cudaStream_t s);
 void launch_norm64(const DevBatch& b, int use_k, int sm_count, cudaStream_t s);
 void launch_write64(const DevBatch& b, int sm_count, cudaStream_t s);
 void launch_gather(const DevBatch& b, int32_t* n_total, int32_t* n_out, double* energy, int32_t* nodes,
                    int32_t* status, double* err_est, int apply_dE, cudaStream_t s);
 
-// polish.cu (fast method: compensated-FP32 recurrence, FP64 matching and norm)
-void launch_newton_df(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_norm_df(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_write_df(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_scale_psi(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_zero_psi(const DevBatch& b, int sm_count, cudaStream_t s);
 void launch_twist64(const DevBatch& b, int sm_count, cudaStream_t s);
 
-// longwin.cu
-void launch_refine_long(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_fallback_long(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_norm_long(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_write_long(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_twist_long(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_norm_fallback(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_refine_mid(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_norm_mid(const DevBatch& b, int sm_count, cudaStream_t s);
+// levelpass.cu
+void levels_set_attributes();
+void launch_order_levels(const DevBatch& b, int sm_count, cudaStream_t s);
+void launch_warp_levels(const DevBatch& b, int sm_count, cudaStream_t s);
+void launch_long_levels(const DevBatch& b, int sm_count, cudaStream_t s);
+void launch_repair(const DevBatch& b, int sm_count, cudaStream_t s);
+void launch_rewrite(const DevBatch& b, int sm_count, cudaStream_t s);
+
+// fragile.cu
+void launch_fragile(const DevBatch& b, int sm_count, cudaStream_t s);
+void launch_fragile_repair(const DevBatch& b, int sm_count, cudaStream_t s);
+void launch_fragile_rewrite(const DevBatch& b, int sm_count, cudaStream_t s);
 
 // adjoint.cu
 // points per CTA of the adjoint (one thread each)

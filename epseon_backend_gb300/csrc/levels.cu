@@ -1,4 +1,5 @@
-// levels.cu -- per-level refinement, normalisation and write-back.
+// levels.cu -- the plain method's per-level refinement, normalisation and
+// write-back, and the results' gather of both methods.
 //
 // Every kernel here is persistent (grid = SMs x resident CTAs) and walks the
 // level slots written by the bracket kernel; the number of slots is read from
@@ -7,8 +8,6 @@
 //  bisect64 : plain method, FP64 bisection on the twisted Sturm count with the
 //             match index k(E) (outer classical turning point), n_bisect halvings
 //             of the scan bracket -- identical arithmetic to the oracle.
-//  refine32 : fast method, safeguarded Cooley-Newton iteration in the FP32
-//             difference form (count + matching residual + norm per pass).
 //  norm64   : FP64 Cooley pass that also fixes the normalisation constants
 //             (sum psi^2 h = 1, psi > 0 next to the inner wall) and the node
 //             count reported for the level.
@@ -26,15 +25,15 @@
 #include <stdint.h>
 
 #include "common.cuh"
-#include "dfpass.cuh"
 #include "launch.h"
-#include "lane32.cuh"
 
 namespace epscu {
 
 namespace {
 
 constexpr int kLevelThreads = 128;
+
+__device__ __forceinline__ bool cancelled(const DevBatch& b) { return b.cancel && *b.cancel; }
 
 // match points stay off the two boundary points (both sides non-empty)
 __device__ __forceinline__ int clamp_inner(const PotMeta& m, int k) { return max(m.i0 + 1, min(k, m.i1 - 1)); }
@@ -171,13 +170,6 @@ __global__ void __launch_bounds__(kLevelThreads) bisect64_kernel(DevBatch b) {
         w.E = __dmul_rn(0.5, __dadd_rn(lo, hi));
         w.iters = m.n_bisect;
         b.levels[slot] = w;
-    }
-}
-
-__global__ void __launch_bounds__(kLaneThreads, kLaneCtasPerSm) refine32_kernel(DevBatch b) {
-    for (int2 unit; next_unit(b, kQRefine32, unit);) {
-        if ((int)(threadIdx.x & 31) >= unit.y) continue;
-        refine32_level(b, unit.x + (threadIdx.x & 31));
     }
 }
 
@@ -331,9 +323,6 @@ int persistent_grid(int sm_count, int per_sm) { return sm_count * per_sm; }
 
 void launch_bisect64(const DevBatch& b, int sm_count, cudaStream_t s) {
     bisect64_kernel<<<persistent_grid(sm_count, 8), kLevelThreads, 0, s>>>(b);
-}
-void launch_refine32(const DevBatch& b, int sm_count, cudaStream_t s) {
-    refine32_kernel<<<persistent_grid(sm_count, kLaneCtasPerSm), kLaneThreads, 0, s>>>(b);
 }
 void launch_norm64(const DevBatch& b, int use_k, int sm_count, cudaStream_t s) {
     norm64_kernel<<<persistent_grid(sm_count, 8), kLevelThreads, 0, s>>>(b, use_k);

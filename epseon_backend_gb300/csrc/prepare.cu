@@ -146,6 +146,10 @@ __global__ void __launch_bounds__(kPrepThreads) prepare_kernel(DevBatch b) {
     last = block_reduce(last, MaxI(), shi);
     const int i0 = first < 1 ? 1 : first;
     const int i1 = last > N - 2 ? N - 2 : last;
+    // a barrier inside the cut-offs that rises above them
+    int steep = 0;
+    for (int i = i0 + tid; i <= i1; i += nt) steep |= dkey0(V[i]) > kt;
+    steep = block_reduce(steep, OrI(), shi);
 
     // argmin on [i0, i1], first occurrence
     unsigned long long bk = kKeyMax;
@@ -246,6 +250,7 @@ __global__ void __launch_bounds__(kPrepThreads) prepare_kernel(DevBatch b) {
         m.n_bisect = K;
         const double kmax = sqrt(2.0 * m.mu * (m.e_cap - vmin));
         if (kmax * h > 1.0) status |= EPSCU_STATUS_UNDER;
+        if (steep) status |= EPSCU_STATUS_STEEP;
         m.status = status;
         m.n_total = 0;
         m.n_out = 0;
@@ -324,7 +329,8 @@ __global__ void __launch_bounds__(1024) level_setup_kernel(DevBatch b) {
 
 // Warp work units for the per-level kernels: each potential's level slots in
 // chunks of 32, potentials in decreasing grid length (the `order` array), so
-// the warp queue hands out the longest work first.  One CTA.
+// the warp queue hands out the longest work first.  (The plain method's.)
+// One CTA.
 __global__ void __launch_bounds__(1024) unit_setup_kernel(DevBatch b) {
     __shared__ int32_t s_u[1024];
     __shared__ int32_t carry;
@@ -445,7 +451,7 @@ __global__ void bracket_kernel(DevBatch b) {
         w.hi0 = w.hi;
         w.j0 = m.i0;
         w.j1 = m.i1;
-        w.pad1 = 0;
+        w.bucket = w.rank = w.pad1 = 0;
         b.levels[m.level_base + s] = w;
     }
 }
@@ -526,46 +532,52 @@ __device__ int2 decay_window(const PotMeta& m, const DevBatch& b, double Eu, flo
     return make_int2(j0, j1);
 }
 
+// The order bucket of a window length: quarter octaves from 16 points up.
+__device__ __forceinline__ int length_bucket(int len) {
+    const int l = 31 - __clz(max(len, 16));
+    return min(kBuckets - 1, 4 * (l - 4) + ((len >> (l - 2)) & 3));
+}
+
 // Decay window of every level slot (fast method), at E_up = hi0 + 2 delta:
 // an energy above every energy the level's passes use (bracket, Newton steps,
-// the fallback's widened bracket), so one window serves all of them.  Levels
-// whose window is longer than the long-window threshold (DevBatch::long_window,
-// else default_long_window of the level count) go to the long list
-// (CTA-per-level passes), those above the middle threshold to the middle list
-// (lane FP32 refinement, then warp-per-level double-float passes); the rest
-// stay on the lane kernels.  One warp per level.
-// (Sharing one window per warp unit would keep the lanes' loads of W
-// warp-wide broadcasts, but the unit's widest window costs more point-updates
-// than the divergent loads: measured slower on the mixed batch.)
-__global__ void __launch_bounds__(128) window_kernel(DevBatch b, int sm_count) {
+// the repair's widened bracket), so one window serves all of them; its match
+// point (the outer turning point at the first energy, on a strip boundary);
+// and its place in the order of the level queues: windows longer than the
+// long-window threshold (DevBatch::long_window, else default_long_window of
+// the level count) on the long list (CTA per level), the rest on the warp
+// list, fragile levels on two lists of their own, by length bucket and rank
+// in it.  One warp per level.
+__global__ void __launch_bounds__(128) window_kernel(DevBatch b) {
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int n_warps = (gridDim.x * blockDim.x) >> 5;
     const int total = b.hdr->total_levels;
-    (void)sm_count;
     const int long_min = b.long_window > 0 ? b.long_window : default_long_window(total);
-    const int mid_w = b.mid_window != 0 ? b.mid_window : kMidWindow;
-    const int mid_min = mid_w <= 0 || !b.mid_list ? 0x7fffffff : mid_w;
+    const int fragile_min = b.long_window > 0 ? b.long_window : default_fragile_window(total);
     for (int slot = warp; slot < total; slot += n_warps) {
         const LevelWork w = b.levels[slot];
-        if (w.status & EPSCU_STATUS_NOTFOUND) continue;
         const PotMeta m = b.meta[w.p];
-        const int2 jw = decay_window(m, b, w.hi0 + 2.0 * m.delta, kWindowDecay);
+        int2 jw = make_int2(m.i0, m.i1);
+        int k = w.k, len = 0, list = kListWarp;  // (a level without a bracket: last on the warp list)
+        if (!(w.status & EPSCU_STATUS_NOTFOUND)) {
+            jw = decay_window(m, b, w.hi0 + 2.0 * m.delta, kWindowDecay);
+            k = match_index(m, b.Msuf, w.E) & ~15;
+            len = jw.y - jw.x;
+            const int s = slot - m.level_base;
+            const bool fragile = (m.status & EPSCU_STATUS_UNDER) ||
+                                 w.n_in_bracket > 1 || (s > 0 && w.hi0 - b.levels[slot - 1].lo0 < kFragileGap) ||
+                                 (s + 1 < m.n_out && b.levels[slot + 1].hi0 - w.lo0 < kFragileGap);
+            list = fragile ? (len > fragile_min ? kListFragileLong : kListFragile)
+                           : (len > long_min ? kListLong : kListWarp);
+        }
         if ((threadIdx.x & 31) == 0) {
-            b.levels[slot].j0 = jw.x;
-            b.levels[slot].j1 = jw.y;
-            if (jw.y - jw.x > long_min && b.long_list) {
-                const int q = atomicAdd(&b.hdr->n_long, 1);
-                if (q < b.max_levels) {
-                    b.long_list[q] = slot;
-                    b.levels[slot].status = w.status | EPSCU_STATUS_LONG;
-                }
-            } else if (jw.y - jw.x > mid_min) {
-                const int q = atomicAdd(&b.hdr->n_mid, 1);
-                if (q < b.max_levels) {
-                    b.mid_list[q] = slot;
-                    b.levels[slot].status = w.status | EPSCU_STATUS_MID;
-                }
-            }
+            const int bucket = list * kBuckets + length_bucket(len);
+            LevelWork* out = b.levels + slot;
+            out->j0 = jw.x;
+            out->j1 = jw.y;
+            out->k = max(jw.x + 1, min(k, jw.y - 1));
+            out->bucket = bucket;
+            out->rank = atomicAdd(&b.hdr->hist[bucket], 1);
+            if (list == kListLong || list == kListFragileLong) out->status = w.status | EPSCU_STATUS_LONG;
         }
     }
 }
@@ -835,12 +847,12 @@ void launch_prepare(const DevBatch& b, cudaStream_t s) {
 
 void launch_level_setup(const DevBatch& b, cudaStream_t s) {
     level_setup_kernel<<<1, 1024, 0, s>>>(b);
-    unit_setup_kernel<<<1, 1024, 0, s>>>(b);
+    if (!b.warp_list) unit_setup_kernel<<<1, 1024, 0, s>>>(b);
     bracket_kernel<<<b.n, 128, 0, s>>>(b);
 }
 
 void launch_window(const DevBatch& b, int sm_count, cudaStream_t s) {
-    window_kernel<<<sm_count * 8, 128, 0, s>>>(b, sm_count);
+    window_kernel<<<sm_count * 8, 128, 0, s>>>(b);
 }
 
 void launch_scan_window(const DevBatch& b, int sm_count, cudaStream_t s) {

@@ -106,8 +106,8 @@ typedef struct epscu_opts {
                             itself runs on the context's stream */
     int32_t tune;        /* 0 = use cached/default launch shape, 1 = autotune */
     int32_t long_window; /* fast method: levels whose window exceeds this many points run
-                            their passes one CTA per level (0: chosen from the number of
-                            levels, 1024 - 8192) */
+                            their passes one CTA per level, the others one warp (0: chosen
+                            from the number of levels, 1024 - 65536) */
     int32_t wait_polls;  /* fast method: bound of each wait of the TMA scan on a staged
                             tile, in non-blocking polls; when it runs out the solve gives up
                             with EPSCU_ERR_TIMEOUT and reports no levels.  0: the default,
@@ -119,11 +119,8 @@ typedef struct epscu_opts {
     int32_t max_iter;    /* fast method: cap on the FP32 refinement passes of a level and
                             on its double-float fallback passes (0: 48 and 96); a level
                             that reaches it carries EPSCU_LEVEL_MAXITER */
-    int32_t mid_window;  /* fast method: > 0: levels whose window exceeds this many points
-                            (and not the long-window threshold) run their double-float passes
-                            one warp per level after the lane FP32 refinement; 0 or < 0: off
-                            (the default: on the 2048-potential batch it did not shorten
-                            the solve) */
+    int32_t mid_window;  /* accepted, without effect: every level below the long-window
+                            threshold runs its passes one warp per level */
     epscu_alloc_fn psi_alloc;  /* EPSCU_MEM_DEVICE with EPSCU_WANT_PSI and result->psi NULL:
                                   the solve reads the wavefunctions' exact size back after
                                   its level set-up and asks psi_alloc for that buffer
@@ -263,9 +260,9 @@ epscu_status epscu_cancel_clear(epscu_ctx* ctx);
 /* Timing of the last solve: per-stage milliseconds (CUDA events on the solve
  * stream) and the counters the roofline uses.  Stages: prepare (set-up and,
  * for the fast method, the scan's decay windows), scan (the scan kernel
- * alone), refine32 (fast: level windows, FP32 refinement and the long-window
- * Newton), polish (Newton, fallback, norm and twist passes; plain: bisection,
- * norm, twist), write (psi write-back). */
+ * alone), refine32 (fast: level windows and the level kernels, psi rows
+ * included), polish (fast: repair and the fragile levels; plain: bisection,
+ * norm, twist), write (plain: psi write-back). */
 typedef struct epscu_stats {
     float ms_prepare, ms_scan, ms_refine32, ms_polish64, ms_write, ms_total;
     int64_t scan_point_updates;    /* trial energies x points of the scan (its window for the fast method) */
@@ -278,27 +275,25 @@ typedef struct epscu_stats {
     int32_t twist_searches;        /* levels re-matched by the twist-index search */
     int32_t norm_redos;            /* norm passes redone at E + dE (fast method) */
     int64_t refine_max_level_updates; /* largest point-updates of one level's FP32
-                                         refinement (fast method; the tail of the
-                                         lane kernel) */
+                                         refinement (fast method) */
     int64_t df_max_level_updates;  /* largest point-updates of one level's double-float
-                                      passes on the lane path (fast method) */
+                                      passes (fast method) */
     int32_t refine_max_iters;      /* most FP32 refinement passes of one level */
     int32_t reserved;
-    /* the long levels' refinement kernel (CTA per level; fast method): its time
-       (EPSCU_STAGE_TIMING only) and its point-updates in FP32 and double-float
-       passes (algorithmic: one grid point of one pass) */
+    /* the level kernels (a warp or a CTA per level; fast method): their time
+       (EPSCU_STAGE_TIMING only), and the CTA levels' point-updates in FP32 and
+       double-float passes (algorithmic: one grid point of one pass) */
     float ms_refine_long;
     int32_t reserved2;
     int64_t long_fp32_point_updates;
     int64_t long_df_point_updates;
-    /* the psi write-back of the fast method: zero_psi writes zeros outside the
-       level windows (its time with EPSCU_STAGE_TIMING only; ms_write is the
-       time of scale_psi, which reads the window's stored pairs and writes the
-       normalised doubles) */
-    float ms_zero_psi;
+    /* the psi write-back of the fast method, inside the level kernels: zeros
+       outside the level windows, and the window points (stored once as pairs,
+       read back and written as the normalised doubles) */
+    float ms_zero_psi;         /* 0 */
     int32_t reserved3;
-    int64_t psi_zero_points;   /* points zero_psi wrote (8 B each) */
-    int64_t psi_window_points; /* window points scale_psi converted (8 B read + 8 B written each) */
+    int64_t psi_zero_points;   /* points zeroed (8 B each) */
+    int64_t psi_window_points; /* window points (8 B stored, 8 B read, 8 B written each) */
 } epscu_stats;
 epscu_status epscu_last_stats(epscu_ctx* ctx, epscu_stats* stats);
 
