@@ -131,6 +131,12 @@ __device__ __forceinline__ void step64(double aE, double w, double& A, double& B
     A = An;
 }
 
+// x < 0 for a number, on the integer pipes: a FP64 comparison costs what a FP64
+// multiply-add does (64 cycles of its SM quarter's pipe a warp on GB300)
+__device__ __forceinline__ bool negative(double x) {
+    return (unsigned long long)__double_as_longlong(x) > 0x8000000000000000ull;
+}
+
 // frexp-style exponent of |m| (m = f 2^e, f in [0.5, 1)) for finite normal m.
 __device__ __forceinline__ int exp_of(double m) {
     const int hi = __double2hiint(m);
@@ -196,46 +202,69 @@ constexpr float kWindowDecay = 36.0f;
 // trial energies per entry of the scan's window table
 constexpr int kScanWinBlock = 128;
 
-// Twisted Sturm count at E with twist index k (identical arithmetic to the
-// oracle's eo_count).
-__device__ __forceinline__ int count64(const PotMeta& m, const double* __restrict__ W, double E, int k) {
-    const double aE = __dmul_rn(m.a, E);
-    int nodes = 0;
-    double A = 1.0, B = 0.0;
-    int s = 0;
-    for (int i = m.i0; i < k; ++i) {
-        const double Ap = A;
-        step64(aE, __ldg(W + i), A, B);
-        nodes += (A < 0.0) != (Ap < 0.0);
+// One side of a twisted Sturm count: the projective state from point `from` up
+// (dir 1) or down (dir -1) to the twist index k, and its sign changes
+// (identical arithmetic to the oracle's eo_count).
+__device__ __forceinline__ int count_side64(const double* __restrict__ W, double aE, int from, int k, int dir, double& A,
+                                            double& B) {
+    A = 1.0;
+    B = 0.0;
+    int nodes = 0, s = 0;
+    bool neg = false;
+    // step64's operations, those of the next point (which do not depend on the
+    // state) between this point's: the chain waits for ~2 FP64 latencies a
+    // step instead of 4
+    double T = __dsub_rn(aE, __ldg(W + from));
+    double f = __dadd_rn(1.0, T), g = __fma_rn(-10.0, T, 2.0);
+    for (int i = from; i != k; i += dir) {
+        const double Tn = __dsub_rn(aE, __ldg(W + i + dir));  // (up to k: inside the grid)
+        const double fB = __dmul_rn(f, B);
+        const double Bn = __dmul_rn(f, A);
+        const double An = __fma_rn(g, A, -fB);
+        f = __dadd_rn(1.0, Tn);
+        g = __fma_rn(-10.0, Tn, 2.0);
+        A = An;
+        B = Bn;
+        const bool n = negative(A);
+        nodes += n != neg;
+        neg = n;
         if (++s == kRenorm) {
             s = 0;
             renorm_pair(A, B);
         }
     }
-    double C = 1.0, D = 0.0;
-    s = 0;
-    for (int i = m.i1; i > k; --i) {
-        const double Cp = C;
-        step64(aE, __ldg(W + i), C, D);
-        nodes += (C < 0.0) != (Cp < 0.0);
-        if (++s == kRenorm) {
-            s = 0;
-            renorm_pair(C, D);
-        }
-    }
-    const double Tk = __dsub_rn(aE, __ldg(W + k));
+    return nodes;
+}
+
+// The count from the two sides' states at k.
+__device__ __forceinline__ int count_join64(double aE, double wk, double A, double B, double C, double D) {
+    const double Tk = __dsub_rn(aE, wk);
     const double fk = __dadd_rn(1.0, Tk);
     const double gk = __fma_rn(-10.0, Tk, 2.0);
     const double AC = __dmul_rn(A, C);
     const double num = __fma_rn(gk, AC, -__dmul_rn(fk, __fma_rn(B, C, __dmul_rn(D, A))));
-    nodes += (num < 0.0) != (AC < 0.0);
-    return nodes;
+    return (num < 0.0) != (AC < 0.0);
+}
+
+// Twisted Sturm count at E with twist index k.
+__device__ __forceinline__ int count64(const PotMeta& m, const double* __restrict__ W, double E, int k) {
+    const double aE = __dmul_rn(m.a, E);
+    double A, B, C, D;
+    int nodes = count_side64(W, aE, m.i0, k, +1, A, B);
+    nodes += count_side64(W, aE, m.i1, k, -1, C, D);
+    return nodes + count_join64(aE, __ldg(W + k), A, B, C, D);
 }
 
 // 1/f for f in [0.4, 4]: FP32 reciprocal refined by two FP64 Newton steps
 // (relative error at the FP64 rounding level).
+// (The two conversions on the integer pipes: exact, and the same rounding.)
 __device__ __forceinline__ double recip64(double f) {
-    double r = (double)__frcp_rn((float)f);
+    const unsigned long long u = (unsigned long long)__double_as_longlong(f);
+    const uint32_t dropped = (uint32_t)u & 0x1fffffffu;
+    uint32_t b = (uint32_t)((u >> 29) - (896ull << 23));  // truncated to a float's bits
+    b += dropped > 0x10000000u || (dropped == 0x10000000u && (b & 1u));
+    const uint32_t x = __float_as_uint(__frcp_rn(__uint_as_float(b)));
+    double r = __hiloint2double((int)((x >> 3) + (896u << 20)), (int)(x << 29));
     r = __fma_rn(r, __fma_rn(-f, r, 1.0), r);
     r = __fma_rn(r, __fma_rn(-f, r, 1.0), r);
     return r;

@@ -325,7 +325,7 @@ void enqueue_pipeline(epscu_ctx* ctx, const DevBatch& b, int method, bool want_p
     if (method == EPSCU_METHOD_PLAIN_FP64) {
         launch_bisect64(b, ctx->sm_count, s);
         rec(3);
-        launch_norm64(b, 0, ctx->sm_count, s);
+        launch_norm64(b, ctx->sm_count, s);
         launch_twist64(b, ctx->sm_count, s);
         rec(4);
         if (want_psi) launch_write64(b, ctx->sm_count, s);

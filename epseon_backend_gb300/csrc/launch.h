@@ -64,19 +64,6 @@ __device__ __forceinline__ int refine_cap(const DevBatch& b) { return b.max_iter
 // double-float fallback passes (bisection from the widened scan bracket)
 __device__ __forceinline__ int fallback_cap(const DevBatch& b) { return 2 * refine_cap(b); }
 
-// Warp-level work queue of the plain method's per-level kernels: units of up to 32
-// consecutive level slots of one potential, longest grids first.  Lane 0
-// takes the next unit and broadcasts it; false when the queue is drained.
-__device__ __forceinline__ bool next_unit(const DevBatch& b, int qid, int2& unit) {
-    int u = 0;
-    if ((threadIdx.x & 31) == 0) u = atomicAdd(&b.hdr->queue[qid], 1);
-    u = __shfl_sync(0xffffffffu, u, 0);
-    if (u >= b.hdr->n_units || u >= b.max_units) return false;
-    unit = b.units[u];
-    return true;
-}
-
-
 // prepare.cu
 void launch_prepare(const DevBatch& b, cudaStream_t s);
 void launch_level_setup(const DevBatch& b, cudaStream_t s);
@@ -106,7 +93,7 @@ void scan32_set_attributes();
 
 // levels.cu
 void launch_bisect64(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_norm64(const DevBatch& b, int use_k, int sm_count, cudaStream_t s);
+void launch_norm64(const DevBatch& b, int sm_count, cudaStream_t s);
 void launch_write64(const DevBatch& b, int sm_count, cudaStream_t s);
 void launch_gather(const DevBatch& b, int32_t* n_total, int32_t* n_out, double* energy, int32_t* nodes,
                    int32_t* status, double* err_est, int apply_dE, cudaStream_t s);

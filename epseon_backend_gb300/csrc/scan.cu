@@ -30,7 +30,7 @@ namespace epscu {
 
 namespace {
 
-constexpr int kScan64Threads = 128;
+constexpr int kScan64Threads = 32;  // (one warp: CTAs spread over the SMs' FP64 pipes)
 
 __global__ void __launch_bounds__(kScan64Threads) scan64_kernel(DevBatch b, int ipp) {
     const int item = blockIdx.x;
