@@ -112,24 +112,54 @@ __global__ void __launch_bounds__(kAdjointPoints) adjoint_kernel(DevBatch b, con
     else gV[offsets[p] + i] = r;
 }
 
-// Explicit layout (stateless adjoint): per-potential arrays on the device.
-__global__ void adjoint_explicit_kernel(int32_t cap, const int64_t* __restrict__ offsets, const int32_t* __restrict__ Ns,
-                                        const double* __restrict__ hs, const int32_t* __restrict__ n_outs,
-                                        const int64_t* __restrict__ psi_offs, const double* __restrict__ psi,
-                                        const double* __restrict__ gE, double* __restrict__ gV) {
+// Explicit layout (stateless adjoint): per-potential arrays on the device, one
+// thread per point, eight rows in flight.  The rows are zero outside their
+// levels' windows (four fifths of the points on the mixed batch), which this
+// entry point does not know: a zero adds nothing, and a warp whose points are
+// all zero in a row skips its FP64 multiply and multiply-add (unless some dL/dE
+// is not finite: its product with zero is not zero).  Multiplying every point
+// the kernel was bound by the FP64 pipe: 1.56 -> 1.19 ms on 256 potentials of
+// 32768 points (3.7 GB of rows).
+constexpr int kExplicitTile = 256;  // dL/dE staged per round
+
+__global__ void __launch_bounds__(256) adjoint_explicit_kernel(
+    int32_t cap, const int64_t* __restrict__ offsets, const int32_t* __restrict__ Ns, const double* __restrict__ hs,
+    const int32_t* __restrict__ n_outs, const int64_t* __restrict__ psi_offs, const double* __restrict__ psi,
+    const double* __restrict__ gE, double* __restrict__ gV) {
+    __shared__ double s_g[kExplicitTile];
     const int p = blockIdx.y;
     const int N = Ns[p];
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= N) return;
+    if ((int)(blockIdx.x * blockDim.x) >= N) return;
     const int n_out = n_outs[p];
-    const double* rows = psi + psi_offs[p] + i;
-    const double* g = gE + (int64_t)p * cap;
+    const double* rows = psi + psi_offs[p] + min(i, N - 1);
     double acc = 0.0;
-    for (int s = 0; s < n_out; ++s) {
-        const double v = __ldg(rows + (int64_t)s * N);
-        acc = fma(g[s] * v, v, acc);
+    for (int t0 = 0; t0 < n_out; t0 += kExplicitTile) {
+        const int nt = min(kExplicitTile, n_out - t0);
+        __syncthreads();  // the previous round's stage is consumed
+        bool odd = false;
+        for (int q = threadIdx.x; q < nt; q += blockDim.x) {
+            const double v = gE[(int64_t)p * cap + t0 + q];
+            s_g[q] = v;
+            odd = odd || (((unsigned long long)__double_as_longlong(v) >> 52) & 0x7ffull) == 0x7ffull;
+        }
+        const bool all = __syncthreads_or(odd) != 0;
+        const double* r = rows + (int64_t)t0 * N;
+        auto add = [&](int q, double v) {
+            if (all || __any_sync(0xffffffffu, ((unsigned long long)__double_as_longlong(v) << 1) != 0ull))
+                acc = fma(s_g[q] * v, v, acc);
+        };
+        int q = 0;
+        for (; q + 7 < nt; q += 8) {
+            double v[8];
+#pragma unroll
+            for (int x = 0; x < 8; ++x) v[x] = __ldg(r + (int64_t)(q + x) * N);
+#pragma unroll
+            for (int x = 0; x < 8; ++x) add(q + x, v[x]);
+        }
+        for (; q < nt; ++q) add(q, __ldg(r + (int64_t)q * N));
     }
-    gV[offsets[p] + i] = acc * hs[p];
+    if (i < N) gV[offsets[p] + i] = acc * hs[p];
 }
 
 }  // namespace
