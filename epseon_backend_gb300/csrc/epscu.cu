@@ -944,32 +944,40 @@ extern "C" epscu_status epscu_tabulate(epscu_ctx* ctx, int32_t n, const int32_t*
     EPSCU_CU(cudaStreamWaitEvent(s, ctx->ev_in, 0));
     const bool dev = (opts.flags & EPSCU_MEM_DEVICE) != 0;
     int64_t total = 0;
+    bool splines = false;
+    std::vector<int32_t> tiles(n + 1);
     // host copies of the per-potential arrays (always host-side per the ABI)
     for (int p = 0; p < n; ++p) {
         if (N[p] < 2) return fail(EPSCU_ERR_INVALID, "grid with fewer than 2 points");
         total = std::max<int64_t>(total, offsets[p] + N[p]);
+        splines = splines || kind[p] == EPSCU_KIND_SPLINE;
+        tiles[p + 1] = tiles[p] + (N[p] + kTabTile - 1) / kTabTile;
     }
     cudaError_t ce = cudaSuccess;
     auto* d_kind = (int32_t*)ctx->get("tab_kind", sizeof(int32_t) * n, &ce);
-    auto* d_par = (double*)ctx->get("tab_par", sizeof(double) * 12 * n, &ce);
     auto* d_off = (int64_t*)ctx->get("tab_off", sizeof(int64_t) * n, &ce);
     auto* d_N = (int32_t*)ctx->get("tab_N", sizeof(int32_t) * n, &ce);
     auto* d_r0 = (double*)ctx->get("tab_r0", sizeof(double) * n, &ce);
     auto* d_r1 = (double*)ctx->get("tab_r1", sizeof(double) * n, &ce);
-    auto* d_scr = (double*)ctx->get("tab_scratch", sizeof(double) * 3 * (size_t)n_knots * n, &ce);
-    if (!d_kind || !d_par || !d_off || !d_N || !d_r0 || !d_r1 || !d_scr) return fail(EPSCU_ERR_NOMEM, "device arena");
+    auto* d_tiles = (int32_t*)ctx->get("tab_tiles", sizeof(int32_t) * (n + 1), &ce);
+    auto* d_scr = (double*)ctx->get("tab_scratch", splines ? sizeof(double) * 4 * (size_t)n_knots * n : 0, &ce);
+    if (!d_kind || !d_off || !d_N || !d_r0 || !d_r1 || !d_tiles || !d_scr) return fail(EPSCU_ERR_NOMEM, "device arena");
     EPSCU_CU(cudaMemcpyAsync(d_kind, kind, sizeof(int32_t) * n, cudaMemcpyHostToDevice, s));
-    EPSCU_CU(cudaMemcpyAsync(d_par, params, sizeof(double) * 12 * n, dev ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice, s));
     EPSCU_CU(cudaMemcpyAsync(d_off, offsets, sizeof(int64_t) * n, cudaMemcpyHostToDevice, s));
     EPSCU_CU(cudaMemcpyAsync(d_N, N, sizeof(int32_t) * n, cudaMemcpyHostToDevice, s));
     EPSCU_CU(cudaMemcpyAsync(d_r0, r_min, sizeof(double) * n, cudaMemcpyHostToDevice, s));
     EPSCU_CU(cudaMemcpyAsync(d_r1, r_max, sizeof(double) * n, cudaMemcpyHostToDevice, s));
+    EPSCU_CU(cudaMemcpyAsync(d_tiles, tiles.data(), sizeof(int32_t) * (n + 1), cudaMemcpyHostToDevice, s));
+    const double* d_par = params;
     double* out = V;
     if (!dev) {
+        auto* par = (double*)ctx->get("tab_par", sizeof(double) * 12 * n, &ce);
         out = (double*)ctx->get("tab_V", sizeof(double) * total, &ce);
-        if (!out) return fail(EPSCU_ERR_NOMEM, "device arena (V)");
+        if (!par || !out) return fail(EPSCU_ERR_NOMEM, "device arena (V)");
+        EPSCU_CU(cudaMemcpyAsync(par, params, sizeof(double) * 12 * n, cudaMemcpyHostToDevice, s));
+        d_par = par;
     }
-    launch_tabulate(n, d_kind, d_par, d_off, d_N, d_r0, d_r1, n_knots, d_scr, out, s);
+    launch_tabulate(n, d_kind, d_par, d_off, d_N, d_r0, d_r1, d_tiles, tiles[n], n_knots, splines, d_scr, out, s);
     EPSCU_CU(cudaGetLastError());
     if (!dev) EPSCU_CU(cudaMemcpyAsync(V, out, sizeof(double) * total, cudaMemcpyDeviceToHost, s));
     EPSCU_CU(cudaEventRecord(ctx->ev_out, s));

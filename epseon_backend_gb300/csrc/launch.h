@@ -69,9 +69,12 @@ void launch_prepare(const DevBatch& b, cudaStream_t s);
 void launch_level_setup(const DevBatch& b, cudaStream_t s);
 void launch_window(const DevBatch& b, int sm_count, cudaStream_t s);
 void launch_scan_window(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_tabulate(int32_t n, const int32_t* kind, const double* params, const int64_t* offsets,
-                     const int32_t* N, const double* r_min, const double* r_max, int32_t n_knots,
-                     double* knot_scratch, double* V, cudaStream_t s);
+
+// tabulate.cu (knot_scratch: 4 n_knots doubles per potential; 6 for the adjoint)
+constexpr int kTabTile = 2048;  // points per CTA; tiles[p]: the first tile of potential p
+void launch_tabulate(int32_t n, const int32_t* kind, const double* params, const int64_t* offsets, const int32_t* N,
+                     const double* r_min, const double* r_max, const int32_t* tiles, int32_t n_tiles, int32_t n_knots,
+                     bool splines, double* knot_scratch, double* V, cudaStream_t s);
 
 void launch_tabulate_adjoint(int32_t n, const int32_t* kind, const double* params, const int64_t* offsets,
                              const int32_t* N, const double* r_min, const double* r_max, int32_t n_knots,
