@@ -79,6 +79,8 @@ struct Header {
     int32_t queue[16];      // work-queue heads of the per-level kernels
     int32_t n_long;         // levels whose window takes the CTA-per-level passes
     int32_t n_warp;         // levels whose window takes the warp-per-level passes
+    int32_t stopped;        // a kernel has seen the host's cancel flag set
+    int32_t n_under;        // potentials on under_list
     int32_t n_fragile;       // fragile levels on lanes, those with long windows,
     int32_t n_fragile_long;
     int32_t n_fragile_fall;  //   those the lane Newton handed over,
@@ -103,7 +105,8 @@ struct Header {
 
 // queue ids of the per-level kernels
 enum { kQBisect64 = 0, kQNorm64, kQWrite64, kQWarpLevels, kQLongLevels, kQRepair, kQWarpRewrite, kQLongRewrite,
-       kQFragileLanes, kQFragileLong, kQFragileRepair, kQFragileRewrite };
+       kQFragileLanes, kQFragileLong, kQFragileRepair, kQFragileRewrite,
+       kQCountStride, kQCountListed };
 
 // internal level flags (not reported: gather keeps the public bits only)
 // the level's final passes ran one CTA per level
@@ -190,8 +193,9 @@ constexpr int kBisectSplit = 16;
 // two dividing kBisectCoarse; 1: no count inside, the level's bracket is the
 // whole cell, which isolates it already)
 constexpr int kBisectSingle = 4;
-// batches of at least this many potentials take the bisection scan (smaller
-// ones have too few CTAs per round to cover its latency; measured on GB300)
+// batches of at least this many potentials scan with a lane per energy (scan.cu;
+// smaller ones have too few energies to cover a lane's march of its window),
+// smaller ones with a group per energy (groupscan.cu)
 constexpr int kBisectMinPotentials = 512;
 
 // e-folds of decay at the ends of the fast method's windows: e^-36 = 2.3e-16,

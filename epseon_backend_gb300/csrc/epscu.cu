@@ -247,6 +247,7 @@ epscu_status epscu_create(int32_t device_ordinal, epscu_ctx** out) {
     c->sm_count = p.multiProcessorCount;
     scan32_set_attributes();
     levels_set_attributes();
+    groupscan_set_attributes();
     *out = c;
     return EPSCU_OK;
 }
@@ -315,8 +316,22 @@ void enqueue_pipeline(epscu_ctx* ctx, const DevBatch& b, int method, bool want_p
         launch_prepare(b, s);
         if (method == EPSCU_METHOD_FAST_FP32C) launch_scan_window(b, ctx->sm_count, s);  // timed with prepare
         rec(1);
-        if (method == EPSCU_METHOD_PLAIN_FP64) launch_scan64(b, s);
-        else if (b.bis_list) launch_bisect_scan(b, shape, ctx->sm_count, s);
+        if (method == EPSCU_METHOD_PLAIN_FP64) {
+            launch_scan64(b, s);
+        } else if (b.under_list) {
+            // a small batch: groups, and beside them the lane scan of the
+            // under-resolved potentials
+            cudaMemsetAsync(b.counts, 0xff, sizeof(int32_t) * (size_t)b.n * b.n_trial, s);  // -1: no count taken
+            cudaStream_t s2 = stage_events ? s : ctx->stream2;
+            if (!stage_events) {
+                cudaEventRecord(ctx->ev_fork, s);
+                cudaStreamWaitEvent(s2, ctx->ev_fork, 0);
+            }
+            launch_scan_under(b, shape, ctx->sm_count, s2);
+            if (!stage_events) cudaEventRecord(ctx->ev_join, s2);
+            launch_group_scan(b, ctx->sm_count, s);
+            if (!stage_events) cudaStreamWaitEvent(s, ctx->ev_join, 0);
+        } else if (b.bis_list) launch_bisect_scan(b, shape, ctx->sm_count, s);
         else launch_scan32(b, shape, ctx->sm_count, s);
         rec(2);
         launch_level_setup(b, s);
@@ -475,6 +490,7 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
     b.fragile_list = b.fragile_long = b.fragile_fall = b.fragile_twist = nullptr;
     b.bis_list = nullptr;
     b.bis_n = nullptr;
+    b.under_list = nullptr;
     b.bis_items = nullptr;
     b.max_bis_items = 0;
     b.Mpre = nullptr;
@@ -496,8 +512,15 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
         const size_t nb = (size_t)(batch->n_trial + kScanWinBlock - 1) / kScanWinBlock;
         b.scan_win = (int2*)ctx->get("scan_win", sizeof(int2) * (size_t)n * nb, &ce);
         if (!b.scan_win) return fail(EPSCU_ERR_NOMEM, "device arena (scan windows)");
-        if (n >= kBisectMinPotentials) {
-            // batches: the bisection scan (counts where they change only)
+        // (wait_polls asks for the TMA scan's waits: the lane scan of every
+        // trial energy on small batches)
+        const bool group_scan = n < kBisectMinPotentials && opts.wait_polls == 0;
+        if (group_scan) {
+            b.under_list = (int32_t*)ctx->get("under_list", sizeof(int32_t) * n, &ce);
+            if (!b.under_list) return fail(EPSCU_ERR_NOMEM, "device arena (under-resolved list)");
+        }
+        if (n >= kBisectMinPotentials || group_scan) {
+            // the bisection scan (counts where they change only)
             b.bis_list = (int32_t*)ctx->get("bis_list", sizeof(int32_t) * (size_t)n * batch->n_trial, &ce);
             b.bis_n = (int32_t*)ctx->get("bis_n", sizeof(int32_t) * (size_t)n, &ce);
             const int64_t items = bisect_max_items(n, batch->n_trial);
@@ -594,7 +617,7 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
         for (const ScanShape& c : cands) {
             EPSCU_CU(cudaMemsetAsync(&b.hdr->queue_scan, 0, sizeof(int32_t), s));
             EPSCU_CU(cudaEventRecord(ctx->ev[6], s));
-            launch_scan32(b, c, ctx->sm_count, s, b.bis_list ? kBisectCoarse : 1);
+            launch_scan32(b, c, ctx->sm_count, s, b.bis_list && !b.under_list ? kBisectCoarse : 1);
             EPSCU_CU(cudaEventRecord(ctx->ev[7], s));
             EPSCU_CU(cudaEventSynchronize(ctx->ev[7]));
             EPSCU_CU(cudaGetLastError());
@@ -766,7 +789,9 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
     // setup, bracket, window, order, the two level kernels, repair, the two
     // fragile kernels, gather
     st.kernel_launches = method == EPSCU_METHOD_FAST_FP32C ? 13 : 9 + (psi_on ? 1 : 0);
-    if (b.bis_list) {  // the plan + count rounds after the coarse scan32
+    if (b.under_list) {  // the group scan's plan, count round and lane scan
+        st.kernel_launches += 3;
+    } else if (b.bis_list) {  // the plan + count rounds after the coarse scan32
         for (int W = kBisectCoarse; W > 1; W /= (W < kBisectSplit ? W : kBisectSplit)) st.kernel_launches += 2;
     }
     if (method == EPSCU_METHOD_PLAIN_FP64) {

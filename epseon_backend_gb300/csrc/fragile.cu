@@ -930,11 +930,11 @@ __device__ __forceinline__ PassDF long_pass32(const Grp& G, const PotMeta& m, co
     return sh.res;
 }
 
-// the host-mapped cancel flag, read by the leader and handed to the group
-// (threads that read it separately could see it change between their reads
+// whether the host asked to stop, looked up by the leader and handed to the
+// group (threads that look separately could see it change between their reads
 // and part at the next barrier)
-__device__ __forceinline__ bool grp_cancelled(const Grp& G, const DevBatch& b, int& slot) {
-    return grp_bcast(G, G.leader() && b.cancel && *b.cancel ? 1 : 0, slot) != 0;
+__device__ __forceinline__ bool grp_cancelled(const Grp& G, const DevBatch& b, int q, int& slot) {
+    return grp_bcast(G, G.leader() && stop_asked(b, (q & 15) == 0) ? 1 : 0, slot) != 0;
 }
 
 // The refinement of a level, in up to three stages:
@@ -1186,7 +1186,7 @@ __global__ void __launch_bounds__(kLongThreads, kLongCtasPerSm) fragile_kernel(D
         LevelWork w = b.levels[slot];
         double* row = psi_row(b, b.meta[w.p], w);
         bool off = false;
-        if (grp_cancelled(G, b, sh.word)) {
+        if (grp_cancelled(G, b, q, sh.word)) {
             w.status |= EPSCU_STATUS_CANCELLED;
         } else {
             refine_cta(G, b, w, false, sh, sh32);
@@ -1237,7 +1237,7 @@ __global__ void __launch_bounds__(kLongThreads, kLongCtasPerSm) fragile_repair_k
         double* row = psi_row(b, b.meta[w.p], w);
         bool off = true;
         if (q < n_fall) {
-            if (grp_cancelled(G, b, sh.word)) {
+            if (grp_cancelled(G, b, q, sh.word)) {
                 w.status |= EPSCU_STATUS_CANCELLED;
                 off = false;
             } else {

@@ -13,8 +13,6 @@ namespace epscu {
 
 namespace {
 
-__device__ __forceinline__ bool cancelled(const DevBatch& b) { return b.cancel && *b.cancel; }
-
 // move the match point to the peak of |psi| when the sampled peak is at least
 // 2^kPeakLog2 (in binary exponent) above |psi_k|
 constexpr int kPeakLog2 = 2;
@@ -160,7 +158,7 @@ __device__ __forceinline__ bool refine32_level(const DevBatch& b, int slot) {
     LevelWork w = b.levels[slot];
     // (long windows take the CTA passes)
     if (w.status & (EPSCU_STATUS_NOTFOUND | EPSCU_STATUS_LONG)) return false;
-    if (pair_first(cancelled(b))) {
+    if (pair_first(stop_asked(b, (slot & 15) == 0))) {
         b.levels[slot].status = w.status | EPSCU_STATUS_CANCELLED;
         return false;
     }

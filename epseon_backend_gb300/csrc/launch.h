@@ -41,9 +41,11 @@ struct DevBatch {
     int32_t* fragile_fall;     // [max_levels]   handed over by the lane Newton
     int32_t* fragile_twist;    // [max_twist]    for the twist-index search
     int32_t* warp_list;        // [max_levels] the other slots (warp-per-level passes), or nullptr
-    int32_t* bis_list;         // [n * n_trial] trial indices of the bisection scan's current round, or
+    int32_t* bis_list;         // [n * n_trial] trial indices of the bisection scan's count round, or
                                // nullptr (every trial energy scanned)
     int32_t* bis_n;            // [n] entries of bis_list per potential
+    int32_t* under_list;       // [n] group scan: the under-resolved potentials, scanned in full by lanes; nullptr:
+                               // every potential scans alike
     int2* bis_items;           // [max_bis_items] (potential, first entry) chunks of a bisection round
     int32_t max_bis_items;
     double* psi;               // compact wavefunctions or nullptr
@@ -63,6 +65,19 @@ constexpr int kRefineMaxIter = 48;        // default cap on a level's FP32 refin
 __device__ __forceinline__ int refine_cap(const DevBatch& b) { return b.max_iter > 0 ? b.max_iter : kRefineMaxIter; }
 // double-float fallback passes (bisection from the widened scan bracket)
 __device__ __forceinline__ int fallback_cap(const DevBatch& b) { return 2 * refine_cap(b); }
+
+// Whether the host asked to stop.  A read of the host-mapped flag goes over the
+// host link, ~2 us each and slower the more warps read at once (a scan that
+// read it per energy spent half its time there, 2432 warps without work took
+// 19 us to find that out), so only the threads that poll read it and tell the
+// others through the header.
+__device__ __forceinline__ bool stop_asked(const DevBatch& b, bool poll) {
+    volatile int32_t* stopped = &b.hdr->stopped;
+    if (*stopped) return true;
+    if (!poll || !b.cancel || !*b.cancel) return false;
+    *stopped = 1;
+    return true;
+}
 
 // prepare.cu
 void launch_prepare(const DevBatch& b, cudaStream_t s);
@@ -89,10 +104,17 @@ struct ScanShape {
     int ctas_per_sm;  // persistent grid = sm_count * ctas_per_sm
 };
 void launch_scan32(const DevBatch& b, const ScanShape& shape, int sm_count, cudaStream_t s, int stride = 1);
+void launch_scan_under(const DevBatch& b, const ScanShape& shape, int sm_count, cudaStream_t s);
+void launch_group_scan(const DevBatch& b, int sm_count, cudaStream_t s);
 void launch_bisect_scan(const DevBatch& b, const ScanShape& shape, int sm_count, cudaStream_t s);
 int64_t bisect_max_items(int n, int n_trial);  // capacity of DevBatch::bis_items
 int scan32_max_tile();
 void scan32_set_attributes();
+
+// groupscan.cu
+void groupscan_set_attributes();
+void launch_count_stride(const DevBatch& b, int stride, int sm_count, cudaStream_t s);
+void launch_count_listed(const DevBatch& b, int chunk, int sm_count, cudaStream_t s);
 
 // levels.cu
 void launch_bisect64(const DevBatch& b, int sm_count, cudaStream_t s);

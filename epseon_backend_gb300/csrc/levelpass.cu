@@ -512,7 +512,7 @@ __global__ void __launch_bounds__(cta_threads<NW>(), ctas_per_sm<NW>()) levels_k
     int32_t* queue = &b.hdr->queue[NW == 1 ? kQWarpLevels : kQLongLevels];
     Tally tally;
     for (;;) {
-        const int2 next = grp_take<NW>(G, b, queue, sh.word);
+        const int2 next = grp_take<NW>(G, b, queue, n, sh.word);
         if (next.x >= n) break;
         const int slot = list[next.x];
         LevelWork w = b.levels[slot];
@@ -648,7 +648,7 @@ __global__ void __launch_bounds__(32 * kCtaWarps, kCtaCtasPerSm) repair_kernel(D
     const int n_fall = min(b.hdr->fallbacks, b.max_levels);
     const int n_twist = min(b.hdr->n_twist, b.max_twist);
     for (;;) {
-        const int2 next = grp_take<NW>(G, b, &b.hdr->queue[kQRepair], sh.word);
+        const int2 next = grp_take<NW>(G, b, &b.hdr->queue[kQRepair], n_fall + n_twist, sh.word);
         const int q = next.x;
         if (q >= n_fall + n_twist) break;
         const bool fall = q < n_fall;
@@ -764,7 +764,7 @@ __global__ void __launch_bounds__(cta_threads<NW>(), ctas_per_sm<NW>()) rewrite_
     const int32_t* list = NW == 1 ? b.warp_list : b.long_list;
     const int n = min(NW == 1 ? b.hdr->n_warp : b.hdr->n_long, b.max_levels);
     for (;;) {
-        const int2 next = grp_take<NW>(G, b, &b.hdr->queue[NW == 1 ? kQWarpRewrite : kQLongRewrite], sh.word);
+        const int2 next = grp_take<NW>(G, b, &b.hdr->queue[NW == 1 ? kQWarpRewrite : kQLongRewrite], n, sh.word);
         if (next.x >= n) break;
         LevelWork w = b.levels[list[next.x]];
         if (NW == 1 && (w.status & EPSCU_STATUS_LONG)) continue;  // (a repaired level: on the long list too)

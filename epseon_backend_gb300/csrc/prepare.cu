@@ -252,6 +252,8 @@ __global__ void __launch_bounds__(kPrepThreads) prepare_kernel(DevBatch b) {
         if (kmax * h > 1.0) status |= EPSCU_STATUS_UNDER;
         if (steep) status |= EPSCU_STATUS_STEEP;
         m.status = status;
+        if (b.under_list && (status & EPSCU_STATUS_UNDER) && !(status & EPSCU_STATUS_BAD))
+            b.under_list[atomicAdd(&b.hdr->n_under, 1)] = p;
         m.n_total = 0;
         m.n_out = 0;
         b.meta[p] = m;
@@ -377,7 +379,7 @@ __global__ void bracket_kernel(DevBatch b) {
         const int v = b.min_level + s;
         int lo = 0, hi = m.n_trial;
         int top = -1;  // trial index of the bracket's upper end (lo when -1)
-        if (!b.bis_list) {
+        if (!b.bis_list || (b.under_list && (m.status & EPSCU_STATUS_UNDER))) {
             while (lo < hi) {
                 const int mid = lo + (hi - lo) / 2;
                 if (c[mid] > v) hi = mid;

@@ -243,7 +243,10 @@ __device__ __forceinline__ void run_down(const float* __restrict__ tb, int T0, i
 }
 
 template <int THREADS, int TILE, int STAGES>
-__global__ void __launch_bounds__(THREADS) scan32_kernel(DevBatch b, int ipp, int n_items, int stride) {
+__global__ void __launch_bounds__(THREADS) scan32_kernel(DevBatch b, int ipp, int n_items, int stride, bool under) {
+    // under: the potentials of under_list only
+    const int32_t* const order = under ? b.under_list : b.order;
+    if (under) n_items = ipp * b.hdr->n_under;
     extern __shared__ __align__(128) unsigned char smem_raw[];
     float2* buf = reinterpret_cast<float2*>(smem_raw);               // STAGES TMA tiles of (w.x, w.y)
     float* conv = reinterpret_cast<float*>(buf + (size_t)STAGES * TILE);  // the converted tile
@@ -274,7 +277,7 @@ __global__ void __launch_bounds__(THREADS) scan32_kernel(DevBatch b, int ipp, in
         __syncthreads();
         const int item = s_item;
         if (item >= n_items || s_abort) break;
-        const int p = b.order[item / ipp];
+        const int p = order[item / ipp];
         // energy blocks highest first: windows (and so the work) grow with
         // the energy, so the longest items of a potential start first
         const int blk = ipp - 1 - item % ipp;
@@ -482,7 +485,8 @@ __global__ void __launch_bounds__(256) bisect_plan_kernel(DevBatch b, int W, int
     // same from run to run, and with it the matching function stored beside
     // each count (atomic list positions made the refinement's first energies,
     // and the final energies' last bits, vary between runs)
-    if (!(m.status & EPSCU_STATUS_BAD)) {
+    const bool lane_scan = b.under_list && (m.status & EPSCU_STATUS_UNDER);
+    if (!(m.status & EPSCU_STATUS_BAD) && !lane_scan) {
         if (W == 0) {
             const int K = (b.n_trial + kBisectCoarse - 1) / kBisectCoarse;
             for (int k = 1 + threadIdx.x; k <= K; k += blockDim.x) list[k - 1] = min(k * kBisectCoarse - 1, last);
@@ -693,7 +697,7 @@ __global__ void __launch_bounds__(kCountThreads) count_list_kernel(DevBatch b) {
 constexpr int kCountCtasPerSm = 8;
 
 template <int THREADS, int TILE, int STAGES>
-void launch_scan32_t(const DevBatch& b, int ctas_per_sm, int sm_count, cudaStream_t s, int stride) {
+void launch_scan32_t(const DevBatch& b, int ctas_per_sm, int sm_count, cudaStream_t s, int stride, bool under) {
     const int ipp = ((b.n_trial + stride - 1) / stride + THREADS - 1) / THREADS;
     const int n_items = ipp * b.n;
     const size_t smem = (size_t)TILE * STAGES * sizeof(float2) + (size_t)TILE * sizeof(float);
@@ -706,7 +710,7 @@ void launch_scan32_t(const DevBatch& b, int ctas_per_sm, int sm_count, cudaStrea
     int grid = sm_count * ctas_per_sm;
     if (grid > n_items) grid = n_items;
     if (grid < 1) grid = 1;
-    kern<<<grid, THREADS, smem, s>>>(b, ipp, n_items, stride);
+    kern<<<grid, THREADS, smem, s>>>(b, ipp, n_items, stride, under);
 }
 
 template <int THREADS, int TILE, int STAGES>
@@ -768,10 +772,13 @@ void launch_bisect_scan(const DevBatch& b, const ScanShape& sh, int sm_count, cu
     }
 }
 
-void launch_scan32(const DevBatch& b, const ScanShape& sh, int sm_count, cudaStream_t s, int stride) {
+namespace {
+
+void launch_scan32_shape(const DevBatch& b, const ScanShape& sh, int sm_count, cudaStream_t s, int stride,
+                         bool under) {
 #define EPSCU_SCAN32_CASE(TH, TI, ST)                                              \
     if (sh.threads == TH && sh.tile == TI && sh.stages == ST) {                    \
-        launch_scan32_t<TH, TI, ST>(b, sh.ctas_per_sm, sm_count, s, stride);       \
+        launch_scan32_t<TH, TI, ST>(b, sh.ctas_per_sm, sm_count, s, stride, under); \
         return;                                                                    \
     }
     EPSCU_SCAN32_CASE(128, 1024, 2)
@@ -785,7 +792,27 @@ void launch_scan32(const DevBatch& b, const ScanShape& sh, int sm_count, cudaStr
     EPSCU_SCAN32_CASE(512, 1024, 4)
     EPSCU_SCAN32_CASE(512, 2048, 3)
 #undef EPSCU_SCAN32_CASE
-    launch_scan32_t<256, 2048, 3>(b, sh.ctas_per_sm, sm_count, s, stride);
+    launch_scan32_t<256, 2048, 3>(b, sh.ctas_per_sm, sm_count, s, stride, under);
+}
+
+}  // namespace
+
+void launch_scan32(const DevBatch& b, const ScanShape& sh, int sm_count, cudaStream_t s, int stride) {
+    launch_scan32_shape(b, sh, sm_count, s, stride, false);
+}
+
+void launch_scan_under(const DevBatch& b, const ScanShape& sh, int sm_count, cudaStream_t s) {
+    launch_scan32_shape(b, sh, sm_count, s, 1, true);
+}
+
+// The bisection scan of a small batch: the coarse grid, then the cells that
+// hold a level, a group of threads per energy (under-resolved potentials
+// excepted: launch_scan_under, beside this).
+void launch_group_scan(const DevBatch& b, int sm_count, cudaStream_t s) {
+    launch_count_stride(b, kBisectCoarse, sm_count, s);
+    static_assert(kBisectSplit == kBisectCoarse, "one round after the coarse grid");
+    bisect_plan_kernel<<<b.n, 256, 0, s>>>(b, kBisectCoarse, kBisectSplit);
+    launch_count_listed(b, kCountEnergies, sm_count, s);
 }
 
 }  // namespace epscu

@@ -5,10 +5,10 @@
 // framework's memory pool or under a strict allocation budget, a process whose
 // allocations are made up front by someone else, or a plugin called from a
 // context where cudaMalloc is not permitted.  For them this entry point runs
-// the trial-energy scan (the same prepare and TMA scan kernels as
-// epscu_solve) on scratch that lives in a file-scope __device__ array of fixed
-// size, allocated by the CUDA runtime when the library is loaded on a device
-// and held until the process exits.  The caller passes the potential and the
+// the trial-energy scan (the same prepare and count kernels as epscu_solve,
+// every trial energy counted) on scratch that lives in a file-scope __device__
+// array of fixed size, allocated by the CUDA runtime when the library is loaded
+// on a device and held until the process exits.  The caller passes the potential and the
 // output buffer (both device pointers) and a stream.
 //
 //  * Maximum grid: kStaticMaxPoints points; longer grids are rejected.
@@ -116,6 +116,7 @@ extern "C" epscu_status epscu_count_levels_static(const double* V, int32_t N, do
             e = cudaGetSymbolAddress(&p, g_static_scan);
             if (e != cudaSuccess) return static_fail(EPSCU_ERR_CUDA, std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e));
             scan32_set_attributes();
+            groupscan_set_attributes();
             g_addr[dev] = static_cast<StaticScanScratch*>(p);
         }
         S = g_addr[dev];
@@ -134,6 +135,7 @@ extern "C" epscu_status epscu_count_levels_static(const double* V, int32_t N, do
     b.counts = counts;
     b.hdr = &S->hdr;
     b.order = S->order;
+    b.under_list = S->order + 1;
     b.n_trial = n_trial;
     b.min_level = 0;
     b.max_level = -1;
@@ -142,7 +144,8 @@ extern "C" epscu_status epscu_count_levels_static(const double* V, int32_t N, do
     static_init_kernel<<<1, 1, 0, s>>>(S, r_min, r_max, mu, e_cap, N, n_trial);
     launch_prepare(b, s);
     const ScanShape shape{256, 2048, 3, 0};
-    launch_scan32(b, shape, sm_count, s);
+    launch_count_stride(b, 1, sm_count, s);
+    launch_scan_under(b, shape, sm_count, s);  // (an under-resolved grid's counts)
     static_finish_kernel<<<1, 1024, 0, s>>>(S, n_trial, counts);
     e = cudaGetLastError();
     if (e != cudaSuccess) return static_fail(EPSCU_ERR_CUDA, cudaGetErrorString(e));
