@@ -35,14 +35,15 @@ constexpr int kRenorm = 32;  // renormalise the projective state every kRenorm s
 struct PotMeta {
     double r_min, r_max, mu, e_cap;  // inputs
     double h, a, e_lo, delta;        // derived (same formulas as the oracle)
-    int64_t off;                     // first element in V64 / W64 / Msuf
+    int64_t off;                     // first element in V64 / W64
     int64_t offf;                    // first element in Wf2 (tile aligned)
     int64_t psi_off;                 // first element of this potential's psi rows
     int32_t N, i0, i1, k_scan;
     int32_t n_bisect, n_trial;
     int32_t n_total, n_out;
     int32_t level_base, status;
-    int32_t pad0, pad1;
+    int32_t prep_done;               // tiles of the prepare kernel that have finished (0 between solves)
+    int32_t pad1;
 };
 
 // One level slot of the refinement stages.
@@ -165,21 +166,6 @@ __device__ __forceinline__ int renorm_pair(double& x, double& y) {
 // E_j = E_lo + (j+1) delta (two roundings, as in the oracle).
 __device__ __forceinline__ double trial_energy(const PotMeta& m, int j) {
     return __dadd_rn(m.e_lo, __dmul_rn((double)(j + 1), m.delta));
-}
-
-// Largest i in [i0, i1] with V_i <= E, by binary search on the suffix minima
-// Msuf_i = min(V_i .. V_{i1}); k_scan when there is none.  Equals the
-// oracle's linear search.
-__device__ __forceinline__ int match_index(const PotMeta& m, const double* __restrict__ Msuf, double E) {
-    const double* M = Msuf + m.off;
-    if (!(M[m.i0] <= E)) return m.k_scan;
-    int lo = m.i0, hi = m.i1;  // invariant: M[lo] <= E
-    while (lo < hi) {
-        const int mid = lo + (hi - lo + 1) / 2;
-        if (M[mid] <= E) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
 }
 
 // bisection scan: the throughput scan on every kBisectCoarse-th trial

@@ -445,6 +445,8 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
         m.r_max = batch->r_max[p];
         m.mu = batch->mu[p];
         m.e_cap = batch->e_cap[p];
+        m.h = (m.r_max - m.r_min) / (double)(N - 1);
+        m.a = m.mu * m.h * m.h / 6.0;
         m.off = off;
         m.offf = total_padded;
         m.N = N;
@@ -471,7 +473,10 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
     b.n = n;
     b.meta = (PotMeta*)ctx->get("meta", sizeof(PotMeta) * n, &ce);
     b.W64 = (double*)ctx->get("W64", sizeof(double) * total_points, &ce);
-    b.Msuf = (double*)ctx->get("Msuf", sizeof(double) * total_points, &ce);
+    b.Bkey = (unsigned long long*)ctx->get("Bkey", sizeof(unsigned long long) * (total_padded / 32), &ce);
+    b.Bsuf = (double*)ctx->get("Bsuf", sizeof(double) * (total_padded / 32), &ce);
+    b.prep_tiles = (int32_t)(total_padded / kPrepTile);
+    b.prep = (PrepTile*)ctx->get("prep", sizeof(PrepTile) * b.prep_tiles, &ce);
     b.Wf2 = method == EPSCU_METHOD_FAST_FP32C ? (float2*)ctx->get("Wf2", sizeof(float2) * total_padded, &ce) : nullptr;
     b.counts = (int32_t*)ctx->get("counts", sizeof(int32_t) * (size_t)n * batch->n_trial, &ce);
     b.gam = method == EPSCU_METHOD_FAST_FP32C ? (float*)ctx->get("gam", sizeof(float) * (size_t)n * batch->n_trial, &ce)
@@ -493,12 +498,12 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
     b.under_list = nullptr;
     b.bis_items = nullptr;
     b.max_bis_items = 0;
-    b.Mpre = nullptr;
+    b.Bpre = nullptr;
     b.Bmin = nullptr;
     if (method == EPSCU_METHOD_FAST_FP32C) {
-        b.Mpre = (double*)ctx->get("Mpre", sizeof(double) * total_points, &ce);
-        b.Bmin = (float*)ctx->get("Bmin", sizeof(float) * (size_t)(total_padded / 32 + 1), &ce);
-        if (!b.Mpre || !b.Bmin) return fail(EPSCU_ERR_NOMEM, "device arena (window bounds)");
+        b.Bpre = (double*)ctx->get("Bpre", sizeof(double) * (total_padded / 32), &ce);
+        b.Bmin = (float*)ctx->get("Bmin", sizeof(float) * (total_padded / 32), &ce);
+        if (!b.Bpre || !b.Bmin) return fail(EPSCU_ERR_NOMEM, "device arena (window bounds)");
         b.long_list = (int32_t*)ctx->get("long_list", sizeof(int32_t) * lv, &ce);
         if (!b.long_list) return fail(EPSCU_ERR_NOMEM, "device arena (long list)");
         b.warp_list = (int32_t*)ctx->get("warp_list", sizeof(int32_t) * lv, &ce);
@@ -531,7 +536,7 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
     }
     int64_t* d_off = (int64_t*)ctx->get("offsets", sizeof(int64_t) * n, &ce);
     int32_t* d_tiles = (int32_t*)ctx->get("adj_tiles", sizeof(int32_t) * (n + 1), &ce);
-    if (ce != cudaSuccess || !b.meta || !b.W64 || !b.Msuf || !b.counts || !b.levels || !b.fallback_list || !b.units ||
+    if (ce != cudaSuccess || !b.meta || !b.W64 || !b.Bkey || !b.Bsuf || !b.prep || !b.counts || !b.levels || !b.fallback_list || !b.units ||
         !b.hdr ||
         !b.order || !d_off || !d_tiles ||
         (method == EPSCU_METHOD_FAST_FP32C && !b.Wf2))
@@ -605,7 +610,6 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
         // time each scan variant on this batch, keep the fastest
         EPSCU_CU(cudaMemcpyAsync(b.meta, hm, sizeof(PotMeta) * n, cudaMemcpyHostToDevice, s));
         EPSCU_CU(cudaMemcpyAsync(b.order, ho, sizeof(int32_t) * n, cudaMemcpyHostToDevice, s));
-        EPSCU_CU(cudaMemsetAsync(b.Wf2, 0, sizeof(float2) * total_padded, s));
         EPSCU_CU(cudaMemsetAsync(b.hdr, 0, sizeof(Header), s));
         launch_prepare(b, s);
         launch_scan_window(b, ctx->sm_count, s);
@@ -651,7 +655,6 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
         if ((e = cudaMemcpyAsync(d_tiles, htile, sizeof(int32_t) * (n + 1), cudaMemcpyHostToDevice, s)) != cudaSuccess)
             return e;
         if ((e = cudaMemsetAsync(b.hdr, 0, sizeof(Header), s)) != cudaSuccess) return e;
-        if (b.Wf2 && (e = cudaMemsetAsync(b.Wf2, 0, sizeof(float2) * total_padded, s)) != cudaSuccess) return e;
         return cudaSuccess;
     };
     auto enqueue_all = [&]() -> cudaError_t {

@@ -970,7 +970,7 @@ __device__ __noinline__ void refine_cta(const Grp& G, const DevBatch& b, LevelWo
     const float2* Wf = b.Wf2 + m.offf;
     const double* W = b.W64 + m.off;
     double lo = w.lo, hi = w.hi, E = w.E, sum = 1.0;
-    int k = grp_bcast(G, G.leader() ? clamp_k(w, match_index(m, b.Msuf, E)) : 0, sh.word);
+    int k = grp_bcast(G, G.leader() ? clamp_k(w, match_index(m, b, E)) : 0, sh.word);
     bool done = false;
     int n_pass = 0, n_pass32 = 0;
     if (!fallback) {
@@ -1095,7 +1095,7 @@ __device__ __noinline__ bool norm_cta(const Grp& G, const DevBatch& b, LevelWork
     }
     int k_row = k;  // the pass whose psi-hat the row holds
     if (r.nodes != w.v) {
-        const int kt = grp_bcast(G, G.leader() ? clamp_k(w, match_index(m, b.Msuf, w.E)) : 0, sh.word);
+        const int kt = grp_bcast(G, G.leader() ? clamp_k(w, match_index(m, b, w.E)) : 0, sh.word);
         PassDF r2 = pass(kt);
         int k2 = kt;
         if (r2.nodes != w.v && r2.peak_log2 >= 1) {

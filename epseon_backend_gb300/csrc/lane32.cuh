@@ -168,7 +168,7 @@ __device__ __forceinline__ bool refine32_level(const DevBatch& b, int slot) {
     double lo = w.lo, hi = w.hi, E = w.E;
     // the level's window (decay window of its bracket)
     auto clamp_w = [&](int kk) { return max(w.j0 + 1, min(kk, w.j1 - 1)); };
-    int k = clamp_w(match_index(m, b.Msuf, E));
+    int k = clamp_w(match_index(m, b, E));
     bool bisect = false, confirming = false, done = false;
     double E_star = E, sum = 1.0;
     int it = 0;

@@ -283,7 +283,7 @@ __device__ __forceinline__ bool norm_df_level(const DevBatch& b, int slot) {
     }
     int k_row = k;  // the pass whose psi-hat the row holds
     if (r.nodes != w.v) {
-        const int kt = clamp_k(w, match_index(m, b.Msuf, w.E));
+        const int kt = clamp_k(w, match_index(m, b, w.E));
         PassDF r2 = pass(kt);
         int k2 = kt;
         if (r2.nodes != w.v && r2.peak_log2 >= 1) {

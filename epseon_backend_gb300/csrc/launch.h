@@ -11,14 +11,28 @@
 
 namespace epscu {
 
+// the prepare kernel's tiles (a divisor of the tile the padded offsets align to)
+constexpr int kPrepTile = 2048;
+struct PrepTile {
+    unsigned long long kall, kin, kmax;  // images of the minimum, the minimum over the interior, the maximum of V
+    int32_t iin;                         // first interior point of the minimum
+    int32_t bad;                         // inf or NaN among the points
+};
+
 struct DevBatch {
     int32_t n;                 // potentials
     PotMeta* meta;             // [n]
     const double* V64;         // concatenated potentials
     double* W64;               // a V (FP64)
-    double* Msuf;              // suffix minima of V on i0..i1
-    double* Mpre;              // prefix minima of V on i0..i1 (fast method), or nullptr
-    float* Bmin;               // minima of W over 32-point blocks (index offf / 32 + block; fast method)
+    // minima over 32-point blocks, at offf / 32 + block: of V (order-preserving
+    // images), of V from the block's start to i1, from i0 to its end, and of W
+    // rounded down (the last two for the fast method, else nullptr)
+    unsigned long long* Bkey;
+    double* Bsuf;
+    double* Bpre;
+    float* Bmin;
+    PrepTile* prep;            // [prep_tiles] summaries of the prepare kernel's tiles
+    int32_t prep_tiles;        // padded points / kPrepTile
     float2* Wf2;               // a V as (hi, lo) floats, tile-aligned per potential
     int32_t* counts;           // [n * n_trial]
     float* gam;                // [n * n_trial] the scan's matching function f_k gamma_k at the counted trial
@@ -59,6 +73,23 @@ struct DevBatch {
     int32_t max_iter;          // cap on FP32 refinement passes (0: 48; fallback passes: twice it)
     double tol;
 };
+
+// Largest i in [i0, i1] with V_i <= E; k_scan when there is none: the last
+// block whose suffix minimum is at or below E, then its points.
+__device__ __forceinline__ int match_index(const PotMeta& m, const DevBatch& b, double E) {
+    const double* S = b.Bsuf + m.offf / 32;
+    int lo = m.i0 >> 5, hi = m.i1 >> 5;  // invariant: S[lo] <= E
+    if (!(S[lo] <= E)) return m.k_scan;
+    while (lo < hi) {
+        const int mid = lo + (hi - lo + 1) / 2;
+        if (S[mid] <= E) lo = mid;
+        else hi = mid - 1;
+    }
+    const double* V = b.V64 + m.off;
+    int i = min((lo << 5) + 31, m.i1);
+    for (const int first = max(lo << 5, m.i0); i > first && !(V[i] <= E);) --i;
+    return i;
+}
 
 constexpr int kWaitPolls = 1 << 22;       // default bound of the TMA scan's mbarrier waits
 constexpr int kRefineMaxIter = 48;        // default cap on a level's FP32 refinement passes

@@ -349,7 +349,7 @@ __device__ __forceinline__ void norm_level(const Grp<NW>& G, const DevBatch& b, 
         }
         if (step == 1 && best.nodes != L.v) {
             const PotMeta m = b.meta[w.p];
-            kk = grp_bcast<NW>(G, G.leader() ? clamp_k(w, match_index(m, b.Msuf, E)) : 0, sh.word);
+            kk = grp_bcast<NW>(G, G.leader() ? clamp_k(w, match_index(m, b, E)) : 0, sh.word);
             continue;  // step 2: the outer turning point
         }
         if (step == 3 && r.nodes == L.v) {

@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(32) bisect64_kernel(DevBatch b, int sms) {
                 mid = __dmul_rn(0.5, __dadd_rn(l, h));
             }
             const double aE = __dmul_rn(m.a, mid);
-            const int k = match_index(m, b.Msuf, mid);
+            const int k = match_index(m, b, mid);
             int count = 0;
             if (d == 0) {
                 if (found) count = count64(m, W, mid, k);
@@ -307,7 +307,7 @@ __global__ void __launch_bounds__(32) norm64_kernel(DevBatch b, int sms) {
         LevelWork w = b.levels[slot];
         if (w.status & (EPSCU_STATUS_NOTFOUND | EPSCU_STATUS_CANCELLED)) continue;
         const PotMeta m = b.meta[w.p];
-        int k = clamp_inner(m, match_index(m, b.Msuf, w.E));
+        int k = clamp_inner(m, match_index(m, b, w.E));
         Pass64 r = cooley64(m, b.W64 + m.off, w.E, k);
         if (r.peak_log2 >= 1) {
             k = clamp_inner(m, r.peak_i);

@@ -17,33 +17,6 @@ namespace {
 
 constexpr int kPrepThreads = 256;
 
-template <typename T, typename Op>
-__device__ T block_reduce(T v, Op op, T* sh) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (lane == 0) sh[warp] = v;
-    __syncthreads();
-    const int nw = blockDim.x >> 5;
-    v = threadIdx.x < nw ? sh[threadIdx.x] : sh[0];
-    if (warp == 0)
-        for (int o = 16; o > 0; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (threadIdx.x == 0) sh[0] = v;
-    __syncthreads();
-    v = sh[0];
-    __syncthreads();
-    return v;
-}
-
-struct MinI {
-    __device__ int operator()(int a, int b) const { return min(a, b); }
-};
-struct MaxI {
-    __device__ int operator()(int a, int b) const { return max(a, b); }
-};
-struct OrI {
-    __device__ int operator()(int a, int b) const { return a | b; }
-};
-
 // An unsigned integer image of a double that orders like the double (for
 // non-NaN values): minima taken on it are exact and need no FP64 instruction.
 constexpr unsigned long long kKeyMax = ~0ull;  // above every image (+inf's image is below it)
@@ -61,9 +34,13 @@ __device__ __forceinline__ unsigned long long dkey0(double x) {
     if ((u << 1) == 0ull) u = 0ull;
     return (u >> 63) ? ~u : (u | 0x8000000000000000ull);
 }
-struct MinU {
-    __device__ unsigned long long operator()(unsigned long long a, unsigned long long b) const { return min(a, b); }
-};
+// the warp's smallest image / largest image, from 32-bit reductions of the halves
+__device__ __forceinline__ unsigned long long warp_min_key(unsigned long long k) {
+    const uint32_t h = __reduce_min_sync(0xffffffffu, (uint32_t)(k >> 32));
+    const uint32_t l = __reduce_min_sync(0xffffffffu, (uint32_t)(k >> 32) == h ? (uint32_t)k : 0xffffffffu);
+    return ((unsigned long long)h << 32) | l;
+}
+__device__ __forceinline__ unsigned long long warp_max_key(unsigned long long k) { return ~warp_min_key(~k); }
 
 // (__double2float_rn(w), __double2float_rn(w - hi)) with integer operations
 // for 2^-60 <= |w| < 2^101 (the conversions otherwise): hi rounds the 52-bit
@@ -93,170 +70,400 @@ __device__ __forceinline__ float2 split_double_rn(double w) {
     return make_float2(__uint_as_float(sgn | hb), lo);
 }
 
-__global__ void __launch_bounds__(kPrepThreads) prepare_kernel(DevBatch b) {
-    __shared__ int shi[32];
-    __shared__ unsigned long long shk[32];
+// ------------------------------------------------------------------ set-up
+// One CTA per tile of kPrepTile points, in one pass over V: W = a V (FP64 and
+// the float pair, zeros in the padding), the minima of the 32-point blocks and
+// the tile's summary.  The last CTA of a potential to finish derives what
+// needs the whole grid from the summaries and from the points of the two tiles
+// that hold the cut-offs; a second kernel, a warp per tile, turns the block
+// minima into suffix and prefix minima.
+//
+// 24 bytes a point are moved (read V, write W twice).  With a CTA per potential,
+// which read V six times and wrote point-wise suffix and prefix minima (16 bytes
+// a point), a potential was one SM's work; both kernels together, before and now:
+//     1 x 2^20 points              6.4 ms   27 us
+//     256 x 2048..65536 points     490 us   71 us
+//     2048 x 2048..65536 points    870 us  390 us  (3 TB/s)
+//     1 x 4096 points               32 us   17 us
+constexpr int kPrepUnroll = kPrepTile / kPrepThreads;
+
+// the potential of tile x (its first tile, kPrepTile padded points each, is at
+// or before x: the last such)
+__device__ __forceinline__ int tile_potential(const DevBatch& b, int x) {
+    const int64_t at = (int64_t)x * kPrepTile;
+    int lo = 0, hi = b.n - 1;
+    while (lo < hi) {
+        const int mid = lo + (hi - lo + 1) / 2;
+        if (b.meta[mid].offf <= at) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// The largest image whose double passes the cut-off test a (V - V_min) <= 1/2
+// (it holds at V_min, is monotone in the image and fails for the NaNs, the
+// images above +inf): a search outward from V_min + 1/(2a), then bisection.
+__device__ unsigned long long cutoff_key(double a, double vmin, unsigned long long kmin) {
+    auto inside = [&](unsigned long long k) { return __dmul_rn(a, __dsub_rn(dkey_inv(k), vmin)) <= 0.5; };
+    unsigned long long lo = kmin, hi = kKeyMax;
+    const unsigned long long g = dkey0(__dadd_rn(vmin, __ddiv_rn(0.5, a)));
+    if (g > lo && g < hi) {
+        unsigned long long step = 1ull;
+        if (inside(g)) {
+            lo = g;
+            while (hi - lo > step) {
+                if (!inside(lo + step)) {
+                    hi = lo + step;
+                    break;
+                }
+                lo += step;
+                step <<= 1;
+            }
+        } else {
+            hi = g;
+            while (hi - lo > step) {
+                if (inside(hi - step)) {
+                    lo = hi - step;
+                    break;
+                }
+                hi -= step;
+                step <<= 1;
+            }
+        }
+    }
+    while (hi - lo > 1ull) {
+        const unsigned long long mid = lo + (hi - lo) / 2;
+        if (inside(mid)) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+// halvings of the trial spacing down to tol (at most 200): the loop
+// w = delta; while w > tol: w /= 2, whose steps are exact
+__device__ __forceinline__ int halvings_to(double delta, double tol) {
+    if (!(delta > tol)) return 0;
+    const unsigned long long ud = (unsigned long long)__double_as_longlong(delta);
+    const unsigned long long ut = (unsigned long long)__double_as_longlong(tol);
+    const int ed = (int)((ud >> 52) & 0x7ff), et = (int)((ut >> 52) & 0x7ff);
+    if (ed == 0x7ff || ed == 0 || et == 0) {  // (infinite, or a denormal halved inexactly)
+        int K = 0;
+        for (double w = delta; w > tol && K < 200; w = __dmul_rn(w, 0.5)) ++K;
+        return K;
+    }
+    const unsigned long long mant = 0xfffffffffffffull;
+    return min(200, ed - et + ((ud & mant) > (ut & mant) ? 1 : 0));
+}
+
+// What the whole grid decides, from the tile summaries (nt of them, at t0).
+__device__ void finish_potential(const DevBatch& b, int p, int nt, const PrepTile* rec) {
+    __shared__ unsigned long long s_k[3][kPrepThreads / 32];
+    __shared__ int s_i[4][kPrepThreads / 32];
     __shared__ unsigned long long s_kt;
-    const int p = b.order[blockIdx.x];  // longest grids first (the tail is the last CTAs)
+    __shared__ double s_delta, s_kmax;
+    __shared__ int s_K;
+    constexpr int nw = kPrepThreads / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     PotMeta m = b.meta[p];
     const double* V = b.V64 + m.off;
     const int N = m.N;
-    const int tid = threadIdx.x, nt = blockDim.x;
 
-    // The per-point comparisons run on order-preserving integer images of the
-    // doubles (dkey0), exact and on the integer pipes: min V and its finiteness,
-    // the cut-off test a (V_i - V_min) <= 1/2 (monotone in V_i, so it holds
-    // exactly up to a threshold image found once per potential by bisection
-    // on the images with the FP64 test itself) and the first argmin; the only
-    // FP64 instruction per point is W = a V.
-    unsigned long long kmin = kKeyMax;
-    int bad = 0;
-    for (int i = tid; i < N; i += nt) {
-        const double v = V[i];
-        if ((((unsigned long long)__double_as_longlong(v) >> 52) & 0x7ffull) == 0x7ffull) bad = 1;  // inf, NaN
-        else kmin = min(kmin, dkey0(v));
-    }
-    kmin = block_reduce(kmin, MinU(), shk);
-    bad = block_reduce(bad, OrI(), shi);
-    const double vmin = dkey_inv(kmin);
-
-    const double h = __ddiv_rn(__dsub_rn(m.r_max, m.r_min), (double)(N - 1));
-    const double a = __ddiv_rn(__dmul_rn(__dmul_rn(m.mu, h), h), 6.0);
-    if (tid == 0) {
-        // the largest image whose double passes the cut-off test (the test
-        // holds at V_min; the images above +inf are NaNs, which fail it)
-        unsigned long long lo = kmin, hi = kKeyMax;
-        while (hi - lo > 1ull) {
-            const unsigned long long mid = lo + (hi - lo) / 2;
-            if (__dmul_rn(a, __dsub_rn(dkey_inv(mid), vmin)) <= 0.5) lo = mid;
-            else hi = mid;
+    // minimum of V, and its first point in the interior (the scan's twist index)
+    unsigned long long kall = kKeyMax, kin = kKeyMax;
+    int iin = N, bad = 0;
+    for (int t = tid; t < nt; t += kPrepThreads) {
+        const PrepTile r = rec[t];
+        kall = min(kall, r.kall);
+        if (r.kin < kin) {
+            kin = r.kin;
+            iin = r.iin;
         }
-        s_kt = lo;
+        bad |= r.bad;
+    }
+    const unsigned long long wall = warp_min_key(kall), win = warp_min_key(kin);
+    const int wi = __reduce_min_sync(0xffffffffu, kin == win ? iin : N);
+    const int wb = __reduce_or_sync(0xffffffffu, bad);
+    if (lane == 0) {
+        s_k[0][warp] = wall;
+        s_k[1][warp] = win;
+        s_i[0][warp] = wi;
+        s_i[1][warp] = wb;
+    }
+    __syncthreads();
+    bad = 0;
+    for (int w = 0; w < nw; ++w) bad |= s_i[1][w];
+    kall = kin = kKeyMax;
+    iin = N;
+    for (int w = 0; w < nw; ++w) {
+        kall = min(kall, s_k[0][w]);
+        if (s_k[1][w] < kin || (s_k[1][w] == kin && s_i[0][w] < iin)) {
+            kin = s_k[1][w];
+            iin = s_i[0][w];
+        }
+    }
+    const double vmin = dkey_inv(kall);
+    if (tid == 0) s_kt = cutoff_key(m.a, vmin, kall);
+    if (tid == 32) {  // (beside it)
+        s_delta = __ddiv_rn(__dsub_rn(m.e_cap, vmin), (double)m.n_trial);
+        s_kmax = sqrt(2.0 * m.mu * (m.e_cap - vmin));
+        s_K = halvings_to(s_delta, b.tol > 0.0 ? b.tol : 1e-12);
     }
     __syncthreads();
     const unsigned long long kt = s_kt;
-    int first = N, last = -1;
-    for (int i = tid; i < N; i += nt) {
-        if (dkey0(V[i]) <= kt) {
-            first = min(first, i);
-            last = max(last, i);
+
+    // the tiles that hold the first and the last point inside the cut-off
+    int ft = nt, lt = -1;
+    for (int t = tid; t < nt; t += kPrepThreads)
+        if (rec[t].kall <= kt) {
+            ft = min(ft, t);
+            lt = max(lt, t);
         }
+    ft = __reduce_min_sync(0xffffffffu, ft);
+    lt = __reduce_max_sync(0xffffffffu, lt);
+    if (lane == 0) {
+        s_i[2][warp] = ft;
+        s_i[3][warp] = lt;
     }
-    first = block_reduce(first, MinI(), shi);
-    last = block_reduce(last, MaxI(), shi);
+    __syncthreads();
+    for (int w = 0; w < nw; ++w) {
+        ft = min(ft, s_i[2][w]);
+        lt = max(lt, s_i[3][w]);
+    }
+    __syncthreads();
+    int first = N, last = -1;
+    if (lt >= 0)
+        for (int x = tid; x < kPrepTile; x += kPrepThreads) {
+            const int i = ft * kPrepTile + x, j = lt * kPrepTile + x;
+            if (i < N && dkey0(V[i]) <= kt) first = min(first, i);
+            if (j < N && dkey0(V[j]) <= kt) last = max(last, j);
+        }
+    first = __reduce_min_sync(0xffffffffu, first);
+    last = __reduce_max_sync(0xffffffffu, last);
+    if (lane == 0) {
+        s_i[0][warp] = first;
+        s_i[1][warp] = last;
+    }
+    __syncthreads();
+    for (int w = 0; w < nw; ++w) {
+        first = min(first, s_i[0][w]);
+        last = max(last, s_i[1][w]);
+    }
     const int i0 = first < 1 ? 1 : first;
     const int i1 = last > N - 2 ? N - 2 : last;
-    // a barrier inside the cut-offs that rises above them
+
+    // a barrier inside the cut-offs that rises above them, and the minima of
+    // the two end tiles over [i0, i1]
     int steep = 0;
-    for (int i = i0 + tid; i <= i1; i += nt) steep |= dkey0(V[i]) > kt;
-    steep = block_reduce(steep, OrI(), shi);
-
-    // argmin on [i0, i1], first occurrence
-    unsigned long long bk = kKeyMax;
-    int bi = N;
-    for (int i = i0 + tid; i <= i1; i += nt) {
-        const unsigned long long k = dkey0(V[i]);
-        if (k < bk) {
-            bk = k;
-            bi = i;
-        }
-    }
-    const unsigned long long gk = block_reduce(bk, MinU(), shk);
-    int cand = (bk == gk) ? bi : N;
-    const int k_scan = block_reduce(cand, MinI(), shi);
-
-    // W = a V in FP64 and as an unevaluated (hi, lo) float pair; zero padding
-    double* W = b.W64 + m.off;
-    float2* Wf = b.Wf2 ? b.Wf2 + m.offf : nullptr;
-    for (int i = tid; i < N; i += nt) {
-        const double w = __dmul_rn(a, V[i]);
-        W[i] = w;
-        if (Wf) Wf[i] = split_double_rn(w);
-    }
-
-    // Suffix minima of V on [i0, i1] (M), and for the fast method prefix
-    // minima (P) and the minima of a V over 32-point blocks clipped to
-    // [i0, i1], rounded down to float (the decay-window bounds).  Coalesced
-    // warp scans over the absolute 32-point blocks B0..B1: each warp owns a
-    // contiguous run of blocks and scans it with shuffles, seeded with the
-    // minimum of the runs to its right (suffix) or left (prefix).  Minima are
-    // taken on an order-preserving integer image of the doubles (exact, and
-    // no FP64 instruction at GB300's 1/64 rate).
-    {
-        const int lane = tid & 31, warp = tid >> 5, nw = nt >> 5;
-        const int B0 = i0 >> 5, B1 = i1 >> 5, nblk = i1 >= i0 ? B1 - B0 + 1 : 0;
-        const int per = (nblk + nw - 1) / nw;
-        const int wb0 = B0 + min(warp * per, nblk), wb1 = B0 + min((warp + 1) * per, nblk);  // [wb0, wb1)
-        __shared__ unsigned long long s_run[32];
-        auto load_key = [&](int B) {
-            const int idx = (B << 5) + lane;
-            return (idx >= i0 && idx <= i1) ? dkey(V[idx]) : kKeyMax;
-        };
-        // this warp's run minimum
-        unsigned long long rm = kKeyMax;
-        for (int B = wb0; B < wb1; ++B) rm = min(rm, load_key(B));
-        for (int o = 16; o > 0; o >>= 1) rm = min(rm, __shfl_xor_sync(0xffffffffu, rm, o));
-        if (lane == 0) s_run[warp] = rm;
-        __syncthreads();
-        double* M = b.Msuf + m.off;
-        unsigned long long carry = kKeyMax;  // the minimum right of this warp's run
-        for (int w = warp + 1; w < nw; ++w) carry = min(carry, s_run[w]);
-        float* Bm = b.Mpre ? b.Bmin + m.offf / 32 : nullptr;
-        for (int B = wb1 - 1; B >= wb0; --B) {
-            unsigned long long k = load_key(B);
-            // inclusive suffix minimum over the lanes (lane l: lanes l..31)
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long y = __shfl_down_sync(0xffffffffu, k, o);
-                if (lane + o < 32) k = min(k, y);
+    unsigned long long ka = kKeyMax, kz = kKeyMax;
+    for (int t = ft + 1 + tid; t < lt; t += kPrepThreads) steep |= rec[t].kmax > kt;
+    if (lt >= 0)
+        for (int x = tid; x < kPrepTile; x += kPrepThreads) {
+            const int i = ft * kPrepTile + x, j = lt * kPrepTile + x;
+            if (i >= i0 && i <= i1) {
+                const unsigned long long k = dkey0(V[i]);
+                ka = min(ka, k);
+                steep |= k > kt;
             }
-            const unsigned long long blk = __shfl_sync(0xffffffffu, k, 0);  // the block's minimum
-            const int idx = (B << 5) + lane;
-            if (idx >= i0 && idx <= i1) M[idx] = dkey_inv(min(k, carry));
-            if (Bm && lane == 0) Bm[B] = __double2float_rd(__dmul_rn(a, dkey_inv(blk)));
-            carry = min(carry, blk);
-        }
-        if (b.Mpre) {
-            double* P = b.Mpre + m.off;
-            carry = kKeyMax;  // the minimum left of this warp's run
-            for (int w = 0; w < warp; ++w) carry = min(carry, s_run[w]);
-            for (int B = wb0; B < wb1; ++B) {
-                unsigned long long k = load_key(B);
-                for (int o = 1; o < 32; o <<= 1) {
-                    const unsigned long long y = __shfl_up_sync(0xffffffffu, k, o);
-                    if (lane >= o) k = min(k, y);
-                }
-                const int idx = (B << 5) + lane;
-                if (idx >= i0 && idx <= i1) P[idx] = dkey_inv(min(k, carry));
-                carry = min(carry, __shfl_sync(0xffffffffu, k, 31));
+            if (j >= i0 && j <= i1) {
+                const unsigned long long k = dkey0(V[j]);
+                kz = min(kz, k);
+                steep |= k > kt;
             }
         }
+    ka = warp_min_key(ka);
+    kz = warp_min_key(kz);
+    steep = __reduce_or_sync(0xffffffffu, steep);
+    if (lane == 0) {
+        s_k[0][warp] = ka;
+        s_k[1][warp] = kz;
+        s_i[2][warp] = steep;
     }
+    __syncthreads();
+    if (tid != 0) return;
+    for (int w = 0; w < nw; ++w) {
+        ka = min(ka, s_k[0][w]);
+        kz = min(kz, s_k[1][w]);
+        steep |= s_i[2][w];
+    }
+    PrepTile* out = const_cast<PrepTile*>(rec);
+    if (lt >= 0) {
+        out[ft].kall = ka;
+        out[lt].kall = kz;  // (one tile: the same minimum)
+    }
+    int status = 0;
+    if (bad) status |= EPSCU_STATUS_BAD | EPSCU_STATUS_NONFINITE;
+    if (i1 - i0 < 2) status |= EPSCU_STATUS_BAD;
+    if (!(m.e_cap > vmin)) status |= EPSCU_STATUS_BAD;
+    m.e_lo = vmin;
+    m.i0 = i0;
+    m.i1 = i1;
+    m.k_scan = i0 <= i1 && iin < N ? iin : i0;
+    m.delta = s_delta;
+    m.n_bisect = s_K;
+    if (s_kmax * m.h > 1.0) status |= EPSCU_STATUS_UNDER;
+    if (steep) status |= EPSCU_STATUS_STEEP;
+    m.status = status;
+    if (b.under_list && (status & EPSCU_STATUS_UNDER) && !(status & EPSCU_STATUS_BAD))
+        b.under_list[atomicAdd(&b.hdr->n_under, 1)] = p;
+    m.n_total = 0;
+    m.n_out = 0;
+    m.prep_done = 0;
+    b.meta[p] = m;
+}
 
+__global__ void __launch_bounds__(kPrepThreads) prepare_kernel(DevBatch b) {
+    __shared__ unsigned long long s_k[3][kPrepThreads / 32];
+    __shared__ int s_i[2][kPrepThreads / 32];
+    __shared__ int s_last;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int p = tile_potential(b, blockIdx.x);
+    const int64_t offf = b.meta[p].offf, off = b.meta[p].off;
+    const int N = b.meta[p].N;
+    const double a = b.meta[p].a;
+    const int t = (int)((int64_t)blockIdx.x - offf / kPrepTile);
+    const int base = t * kPrepTile;
+    const double* V = b.V64 + off;
+    double* W = b.W64 + off;
+    float2* Wf = b.Wf2 ? b.Wf2 + offf : nullptr;
+
+    double v[kPrepUnroll];
+#pragma unroll
+    for (int u = 0; u < kPrepUnroll; ++u) {
+        const int i = base + u * kPrepThreads + tid;
+        v[u] = i < N ? V[i] : 0.0;
+    }
+    // the comparisons run on order-preserving integer images of the doubles
+    // (dkey0), exact and on the integer pipes; the only FP64 instruction per
+    // point is W = a V
+    unsigned long long kall = kKeyMax, kin = kKeyMax, kmax = 0ull;
+    int iin = N, bad = 0;
+#pragma unroll
+    for (int u = 0; u < kPrepUnroll; ++u) {
+        const int i = base + u * kPrepThreads + tid;
+        const bool on = i < N;
+        const double w = __dmul_rn(a, v[u]);
+        if (on) W[i] = w;
+        if (Wf) Wf[i] = on ? split_double_rn(w) : make_float2(0.0f, 0.0f);
+        unsigned long long k = kKeyMax;
+        if (on) {
+            k = dkey0(v[u]);
+            if ((((unsigned long long)__double_as_longlong(v[u]) >> 52) & 0x7ffull) == 0x7ffull) bad = 1;  // inf, NaN
+            kmax = max(kmax, k);
+        }
+        const unsigned long long blk = warp_min_key(k);
+        if (lane == 0 && on) b.Bkey[(offf + i) >> 5] = blk;
+        kall = min(kall, blk);
+        // the first interior point of the smallest image (i grows with u)
+        const unsigned long long ki = i >= 1 && i <= N - 2 ? k : kKeyMax;
+        if (ki < kin) {
+            kin = ki;
+            iin = i;
+        }
+    }
+    if (base >= N) return;  // (padding only; uniform over the CTA)
+    const unsigned long long win = warp_min_key(kin), wmax = warp_max_key(kmax);
+    const int wi = __reduce_min_sync(0xffffffffu, kin == win ? iin : N);
+    bad = __reduce_or_sync(0xffffffffu, bad);
+    if (lane == 0) {
+        s_k[0][warp] = kall;
+        s_k[1][warp] = win;
+        s_k[2][warp] = wmax;
+        s_i[0][warp] = wi;
+        s_i[1][warp] = bad;
+    }
+    __syncthreads();
+    const int nt = (N + kPrepTile - 1) / kPrepTile;
+    PrepTile* rec = b.prep + offf / kPrepTile;
     if (tid == 0) {
-        int status = 0;
-        if (bad) status |= EPSCU_STATUS_BAD | EPSCU_STATUS_NONFINITE;
-        if (i1 - i0 < 2) status |= EPSCU_STATUS_BAD;
-        if (!(m.e_cap > vmin)) status |= EPSCU_STATUS_BAD;
-        m.h = h;
-        m.a = a;
-        m.e_lo = vmin;
-        m.i0 = i0;
-        m.i1 = i1;
-        m.k_scan = k_scan < N ? k_scan : i0;
-        m.delta = __ddiv_rn(__dsub_rn(m.e_cap, vmin), (double)m.n_trial);
-        const double tol = b.tol > 0.0 ? b.tol : 1e-12;
-        int K = 0;
-        for (double w = m.delta; w > tol && K < 200; w = __dmul_rn(w, 0.5)) ++K;
-        m.n_bisect = K;
-        const double kmax = sqrt(2.0 * m.mu * (m.e_cap - vmin));
-        if (kmax * h > 1.0) status |= EPSCU_STATUS_UNDER;
-        if (steep) status |= EPSCU_STATUS_STEEP;
-        m.status = status;
-        if (b.under_list && (status & EPSCU_STATUS_UNDER) && !(status & EPSCU_STATUS_BAD))
-            b.under_list[atomicAdd(&b.hdr->n_under, 1)] = p;
-        m.n_total = 0;
-        m.n_out = 0;
-        b.meta[p] = m;
+        PrepTile r{kKeyMax, kKeyMax, 0ull, N, 0};
+        for (int w = 0; w < kPrepThreads / 32; ++w) {
+            r.kall = min(r.kall, s_k[0][w]);
+            r.kmax = max(r.kmax, s_k[2][w]);
+            r.bad |= s_i[1][w];
+            if (s_k[1][w] < r.kin || (s_k[1][w] == r.kin && s_i[0][w] < r.iin)) {
+                r.kin = s_k[1][w];
+                r.iin = s_i[0][w];
+            }
+        }
+        rec[t] = r;
+        __threadfence();
+        s_last = nt == 1 || atomicAdd(&b.meta[p].prep_done, 1) == nt - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (s_last) finish_potential(b, p, nt, rec);
+}
+
+// Suffix and prefix minima of V over the 32-point blocks of [i0, i1] (the
+// minimum from a block's start to i1, and from i0 to its end), and for the
+// fast method the block minima of a V rounded down to float (the decay-window
+// bounds).  One warp per tile of 64 blocks; what lies beyond the tile comes
+// from the tile summaries.
+__global__ void __launch_bounds__(128) block_minima_kernel(DevBatch b, int n_tiles) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int x = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (x >= n_tiles) return;
+    const int p = tile_potential(b, x);
+    const PotMeta& m = b.meta[p];
+    const int t = (int)((int64_t)x - m.offf / kPrepTile);
+    if (t * kPrepTile >= m.N || (m.status & EPSCU_STATUS_BAD)) return;
+    const int i0 = m.i0, i1 = m.i1;
+    const int ft = i0 / kPrepTile, lt = i1 / kPrepTile;
+    if (t < ft || t > lt) return;
+    const PrepTile* rec = b.prep + m.offf / kPrepTile;
+    unsigned long long right = kKeyMax, left = kKeyMax;
+    for (int q = t + 1 + lane; q <= lt; q += 32) right = min(right, rec[q].kall);
+    for (int q = ft + lane; q < t; q += 32) left = min(left, rec[q].kall);
+    right = warp_min_key(right);
+    left = warp_min_key(left);
+    const int64_t B0 = m.offf / 32;
+    const double* V = b.V64 + m.off;
+    const double a = m.a;
+    constexpr int kPer = kPrepTile / 32 / 32;  // blocks per lane
+    unsigned long long k[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int B = t * (kPrepTile / 32) + u * 32 + lane;
+        k[u] = B >= (i0 >> 5) && B <= (i1 >> 5) ? b.Bkey[B0 + B] : kKeyMax;
+        // the blocks that the cut-offs cut: over their points inside
+        for (int end = 0; end < 2; ++end) {
+            const int Bc = (end ? i1 : i0) >> 5;
+            if (Bc < t * (kPrepTile / 32) + u * 32 || Bc >= t * (kPrepTile / 32) + u * 32 + 32) continue;  // (uniform)
+            const int i = (Bc << 5) + lane;
+            const unsigned long long kc = warp_min_key(i >= i0 && i <= i1 ? dkey0(V[i]) : kKeyMax);
+            if (B == Bc) k[u] = kc;
+        }
+    }
+    unsigned long long suf[kPer], pre[kPer];
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        suf[u] = pre[u] = k[u];
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_down_sync(full, suf[u], o), z = __shfl_up_sync(full, pre[u], o);
+            if (lane + o < 32) suf[u] = min(suf[u], y);
+            if (lane >= o) pre[u] = min(pre[u], z);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        pre[u] = min(pre[u], left);
+        left = __shfl_sync(full, pre[u], 31);
+    }
+#pragma unroll
+    for (int u = kPer - 1; u >= 0; --u) {
+        suf[u] = min(suf[u], right);
+        right = __shfl_sync(full, suf[u], 0);
+    }
+#pragma unroll
+    for (int u = 0; u < kPer; ++u) {
+        const int B = t * (kPrepTile / 32) + u * 32 + lane;
+        if (B < (i0 >> 5) || B > (i1 >> 5)) continue;
+        b.Bsuf[B0 + B] = dkey_inv(suf[u]);
+        if (b.Bpre) {
+            b.Bpre[B0 + B] = dkey_inv(pre[u]);
+            b.Bmin[B0 + B] = __double2float_rd(__dmul_rn(a, dkey_inv(k[u])));
+        }
     }
 }
 
@@ -478,12 +685,23 @@ __device__ int2 decay_window(const PotMeta& m, const DevBatch& b, double Eu, flo
     const unsigned full = 0xffffffffu;
     const float aEu = __double2float_ru(m.a * Eu);
     const float* Bm = b.Bmin + m.offf / 32;
-    const int t_out = match_index(m, b.Msuf, Eu);
-    int t_in;
+    const int B_first = m.i0 >> 5, B_last = m.i1 >> 5;
+    // the blocks of the outermost points at or below Eu: the last one whose
+    // suffix minimum is, the first one whose prefix minimum is
+    int t_out = m.k_scan >> 5, t_in = B_last;
     {
-        // first i with min(V_i0 .. V_i) <= Eu (the prefix minima do not increase)
-        const double* P = b.Mpre + m.off;
-        int lo = m.i0, hi = m.i1;
+        const double* S = b.Bsuf + m.offf / 32;
+        if (S[B_first] <= Eu) {
+            int lo = B_first, hi = B_last;
+            while (lo < hi) {
+                const int mid = lo + (hi - lo + 1) / 2;
+                if (S[mid] <= Eu) lo = mid;
+                else hi = mid - 1;
+            }
+            t_out = lo;
+        }
+        const double* P = b.Bpre + m.offf / 32;
+        int lo = B_first, hi = B_last;
         while (lo < hi) {
             const int mid = lo + (hi - lo) / 2;
             if (P[mid] <= Eu) hi = mid;
@@ -491,45 +709,45 @@ __device__ int2 decay_window(const PotMeta& m, const DevBatch& b, double Eu, flo
         }
         t_in = lo;
     }
-    const int B_first = m.i0 >> 5, B_last = m.i1 >> 5;
     auto block_decay = [&](int B) {
         const int n = min((B << 5) + 31, m.i1) - max(B << 5, m.i0) + 1;
         return (float)n * acoshf(1.0f + 6.0f * fmaxf(Bm[B] - aEu, 0.0f));
     };
-    int j1 = m.i1;
-    float X = 0.0f;
-    for (int B0 = (t_out >> 5) + 1; B0 <= B_last; B0 += 32) {
-        const int B = B0 + lane;
-        float s = B <= B_last ? block_decay(B) : 0.0f;
+    // The block, going dir from B0, at which the e-folds summed from there on
+    // reach decay (none: -1).  Four runs of 32 blocks at a time: their loads and
+    // scans overlap, the sums are taken run by run (a run at a time waits ~700
+    // cycles for each load: 0.33 ms a window kernel on a 2^20-point grid).
+    auto reach = [&](int B0, int dir) {
+        constexpr int kRuns = 4;
+        const int n_blk = dir > 0 ? B_last - B0 + 1 : B0 - B_first + 1;
+        float X = 0.0f;
+        for (int q0 = 0; q0 < n_blk; q0 += 32 * kRuns) {
+            float s[kRuns];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float y = __shfl_up_sync(full, s, o);
-            if (lane >= o) s += y;
-        }
-        const unsigned hit = __ballot_sync(full, B <= B_last && X + s >= decay);
-        if (hit) {
-            j1 = min(((B0 + __ffs(hit) - 1) << 5) + 31, m.i1);
-            break;
-        }
-        X += __shfl_sync(full, s, 31);
-    }
-    int j0 = m.i0;
-    X = 0.0f;
-    for (int B0 = (t_in >> 5) - 1; B0 >= B_first; B0 -= 32) {
-        const int B = B0 - lane;
-        float s = B >= B_first ? block_decay(B) : 0.0f;
+            for (int u = 0; u < kRuns; ++u) {
+                const int q = q0 + 32 * u + lane;
+                s[u] = q < n_blk ? block_decay(B0 + dir * q) : 0.0f;
+            }
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const float y = __shfl_up_sync(full, s, o);
-            if (lane >= o) s += y;
+            for (int o = 1; o < 32; o <<= 1) {
+#pragma unroll
+                for (int u = 0; u < kRuns; ++u) {
+                    const float y = __shfl_up_sync(full, s[u], o);
+                    if (lane >= o) s[u] += y;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kRuns; ++u) {
+                const unsigned hit = __ballot_sync(full, q0 + 32 * u + lane < n_blk && X + s[u] >= decay);
+                if (hit) return B0 + dir * (q0 + 32 * u + __ffs(hit) - 1);
+                X += __shfl_sync(full, s[u], 31);
+            }
         }
-        const unsigned hit = __ballot_sync(full, B >= B_first && X + s >= decay);
-        if (hit) {
-            j0 = max((B0 - (__ffs(hit) - 1)) << 5, m.i0);
-            break;
-        }
-        X += __shfl_sync(full, s, 31);
-    }
+        return -1;
+    };
+    const int b_out = reach(t_out + 1, 1), b_in = reach(t_in - 1, -1);
+    const int j1 = b_out >= 0 ? min((b_out << 5) + 31, m.i1) : m.i1;
+    const int j0 = b_in >= 0 ? max(b_in << 5, m.i0) : m.i0;
     if (j1 - j0 < 4) return make_int2(m.i0, m.i1);
     return make_int2(j0, j1);
 }
@@ -562,7 +780,7 @@ __global__ void __launch_bounds__(128) window_kernel(DevBatch b) {
         int k = w.k, len = 0, list = kListWarp;  // (a level without a bracket: last on the warp list)
         if (!(w.status & EPSCU_STATUS_NOTFOUND)) {
             jw = decay_window(m, b, w.hi0 + 2.0 * m.delta, kWindowDecay);
-            k = match_index(m, b.Msuf, w.E) & ~15;
+            k = match_index(m, b, w.E) & ~15;
             len = jw.y - jw.x;
             const int s = slot - m.level_base;
             const bool fragile = (m.status & EPSCU_STATUS_UNDER) ||
@@ -606,7 +824,8 @@ __global__ void __launch_bounds__(128) scan_window_kernel(DevBatch b, int n_blk)
 }  // namespace
 
 void launch_prepare(const DevBatch& b, cudaStream_t s) {
-    prepare_kernel<<<b.n, kPrepThreads, 0, s>>>(b);
+    prepare_kernel<<<b.prep_tiles, kPrepThreads, 0, s>>>(b);
+    block_minima_kernel<<<(b.prep_tiles + 3) / 4, 128, 0, s>>>(b, b.prep_tiles);
 }
 
 void launch_level_setup(const DevBatch& b, cudaStream_t s) {

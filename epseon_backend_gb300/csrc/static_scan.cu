@@ -38,7 +38,9 @@ constexpr int kStaticMaxPoints = 65536;  // multiple of the scan's largest tile 
 
 struct StaticScanScratch {
     double W64[kStaticMaxPoints];
-    double Msuf[kStaticMaxPoints];
+    unsigned long long Bkey[kStaticMaxPoints / 32];
+    double Bsuf[kStaticMaxPoints / 32];
+    PrepTile prep[kStaticMaxPoints / kPrepTile];
     float2 Wf2[kStaticMaxPoints];
     PotMeta meta;
     Header hdr;
@@ -57,6 +59,8 @@ __global__ void static_init_kernel(StaticScanScratch* s, double r_min, double r_
     m.r_max = r_max;
     m.mu = mu;
     m.e_cap = e_cap;
+    m.h = __ddiv_rn(__dsub_rn(r_max, r_min), (double)(N - 1));
+    m.a = __ddiv_rn(__dmul_rn(__dmul_rn(mu, m.h), m.h), 6.0);
     m.off = 0;
     m.offf = 0;
     m.N = N;
@@ -130,7 +134,10 @@ extern "C" epscu_status epscu_count_levels_static(const double* V, int32_t N, do
     b.meta = &S->meta;
     b.V64 = V;
     b.W64 = S->W64;
-    b.Msuf = S->Msuf;
+    b.Bkey = S->Bkey;
+    b.Bsuf = S->Bsuf;
+    b.prep = S->prep;
+    b.prep_tiles = (N + kPrepTile - 1) / kPrepTile;
     b.Wf2 = S->Wf2;
     b.counts = counts;
     b.hdr = &S->hdr;
