@@ -27,7 +27,7 @@ namespace epscu {
 
 // the fast method's level lists (LevelWork::bucket / kBuckets), each ordered by
 // window-length classes (quarter octaves)
-enum { kListWarp = 0, kListLong, kListFragile, kListFragileLong, kLists };
+enum { kListWarp = 0, kListLong, kListFragile, kListFragileLong, kListCluster, kLists };
 constexpr int kBuckets = 64;
 constexpr int kRenorm = 32;  // renormalise the projective state every kRenorm steps
 
@@ -80,6 +80,7 @@ struct Header {
     int32_t queue[16];      // work-queue heads of the per-level kernels
     int32_t n_long;         // levels whose window takes the CTA-per-level passes
     int32_t n_warp;         // levels whose window takes the warp-per-level passes
+    int32_t n_cluster;      // levels whose window takes the passes of a cluster of CTAs
     int32_t stopped;        // a kernel has seen the host's cancel flag set
     int32_t n_under;        // potentials on under_list
     int32_t n_fragile;       // fragile levels on lanes, those with long windows,
@@ -107,11 +108,13 @@ struct Header {
 // queue ids of the per-level kernels
 enum { kQBisect64 = 0, kQNorm64, kQWrite64, kQWarpLevels, kQLongLevels, kQRepair, kQWarpRewrite, kQLongRewrite,
        kQFragileLanes, kQFragileLong, kQFragileRepair, kQFragileRewrite,
-       kQCountStride, kQCountListed };
+       kQCountStride, kQCountListed, kQClusterLevels, kQClusterRewrite };
 
 // internal level flags (not reported: gather keeps the public bits only)
 // the level's final passes ran one CTA per level
 #define EPSCU_STATUS_LONG 0x20000
+// ... and those a cluster of CTAs
+#define EPSCU_STATUS_CLUSTER 0x80000
 // (fragile.cu) the lane Newton handed the level over: its refinement, norm pass
 // and rewrite run on a CTA (the lane passes skip it)
 #define EPSCU_STATUS_FALLBACK 0x10000

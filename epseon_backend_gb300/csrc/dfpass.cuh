@@ -13,7 +13,13 @@ namespace epscu {
 // Windows longer than a threshold take a CTA per level, the others a warp.  A
 // warp per level costs the fewest instructions (no barriers, one scan), but a
 // level's march is then 32 threads' and a batch of few levels leaves the GPU
-// idle, so the threshold falls with the number of levels.
+// idle, so the threshold falls with the number of levels.  Solve times by
+// threshold (Morse grids; the rule's choice in brackets):
+//     levels x points     1024   4096  16384  65536
+//        56 x 4096       [330]   398    401    411 us
+//      3680 x 16384      1403  [1073]  1331   1330 us
+//     14128 x 32768      6855   6281  [5233] 22050 us
+//        37 x 65536     [1041]  1042   1721   3010 us
 // DevBatch::long_window > 0 overrides it.
 constexpr int kLongWindow = 65536;
 constexpr int kLongWindowLevels = 45000;
@@ -23,6 +29,23 @@ __host__ __device__ __forceinline__ int default_long_window(int total_levels) {
     int w = kMinLongWindow;
     while (w < kLongWindow && (long long)w * kLongWindowLevels < (long long)kLongWindow * total_levels) w <<= 1;
     return w;
+}
+
+// Windows longer than a second threshold take a cluster of four CTAs per level:
+// 1024 threads on one march instead of 256, where the longest of a few levels'
+// marches is what a solve waits for (280 levels on 2^20 points: 5.8 -> 2.0 ms
+// of level passes; 37 levels on 65536 points, the solve 674 -> 487 us; 333
+// levels on 65536 points with the threshold at 16384 instead of 32768: 888
+// instead of 693 us, so it too rises with the number of levels).  Batches of
+// more than kClusterPotentials potentials have levels enough for the CTAs.
+constexpr int kMinClusterWindow = 16384;
+constexpr int kClusterLevels = 256;
+constexpr int kClusterPotentials = 16;
+
+__host__ __device__ __forceinline__ int default_cluster_window(int total_levels) {
+    long long w = kMinClusterWindow;
+    while (w < (1ll << 30) && w * kClusterLevels < (long long)kMinClusterWindow * total_levels) w <<= 1;
+    return (int)w;
 }
 
 // The threshold of the fragile levels' CTA passes (fragile.cu), which cost ~3x

@@ -355,15 +355,13 @@ void enqueue_pipeline(epscu_ctx* ctx, const DevBatch& b, int method, bool want_p
             launch_fragile(b, ctx->sm_count, ctx->stream2);
             launch_fragile_repair(b, ctx->sm_count, ctx->stream2);
             cudaEventRecord(ctx->ev_join, ctx->stream2);
-            launch_long_levels(b, ctx->sm_count, s);
-            launch_warp_levels(b, ctx->sm_count, s);
+            launch_levels(b, ctx->sm_count, s);
             launch_repair(b, ctx->sm_count, s);
             cudaStreamWaitEvent(s, ctx->ev_join, 0);
         } else {
             // stage timing: one stream, stages in sequence
             rec(8);
-            launch_long_levels(b, ctx->sm_count, s);
-            launch_warp_levels(b, ctx->sm_count, s);
+            launch_levels(b, ctx->sm_count, s);
             rec(9);
             rec(3);
             launch_repair(b, ctx->sm_count, s);
@@ -491,6 +489,7 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
     b.order = (int32_t*)ctx->get("order", sizeof(int32_t) * n, &ce);
     b.scan_win = nullptr;
     b.long_list = nullptr;
+    b.cluster_list = nullptr;
     b.warp_list = nullptr;
     b.fragile_list = b.fragile_long = b.fragile_fall = b.fragile_twist = nullptr;
     b.bis_list = nullptr;
@@ -506,6 +505,10 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
         if (!b.Bpre || !b.Bmin) return fail(EPSCU_ERR_NOMEM, "device arena (window bounds)");
         b.long_list = (int32_t*)ctx->get("long_list", sizeof(int32_t) * lv, &ce);
         if (!b.long_list) return fail(EPSCU_ERR_NOMEM, "device arena (long list)");
+        if (max_N > kMinClusterWindow && n <= kClusterPotentials) {
+            b.cluster_list = (int32_t*)ctx->get("cluster_list", sizeof(int32_t) * lv, &ce);
+            if (!b.cluster_list) return fail(EPSCU_ERR_NOMEM, "device arena (cluster list)");
+        }
         b.warp_list = (int32_t*)ctx->get("warp_list", sizeof(int32_t) * lv, &ce);
         if (!b.warp_list) return fail(EPSCU_ERR_NOMEM, "device arena (warp list)");
         b.fragile_list = (int32_t*)ctx->get("fragile_list", sizeof(int32_t) * lv, &ce);

@@ -49,6 +49,8 @@ struct DevBatch {
     Header* hdr;
     int32_t* order;            // [n] potentials by decreasing cost
     int2* scan_win;            // [n * ceil(n_trial / kScanWinBlock)] scan windows, or nullptr (full grid)
+    int32_t* cluster_list;     // [max_levels] slots with the longest windows (a cluster of CTAs each), or nullptr:
+                               // none can be that long
     int32_t* long_list;        // [max_levels] slots with long windows (CTA-per-level passes), or nullptr
     int32_t* fragile_list;     // [max_levels] fragile levels (fragile.cu): a lane each, or nullptr
     int32_t* fragile_long;     // [max_levels]   long windows, a CTA each
@@ -159,8 +161,7 @@ void launch_twist64(const DevBatch& b, int sm_count, cudaStream_t s);
 // levelpass.cu
 void levels_set_attributes();
 void launch_order_levels(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_warp_levels(const DevBatch& b, int sm_count, cudaStream_t s);
-void launch_long_levels(const DevBatch& b, int sm_count, cudaStream_t s);
+void launch_levels(const DevBatch& b, int sm_count, cudaStream_t s);
 void launch_repair(const DevBatch& b, int sm_count, cudaStream_t s);
 void launch_rewrite(const DevBatch& b, int sm_count, cudaStream_t s);
 

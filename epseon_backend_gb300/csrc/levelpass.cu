@@ -4,7 +4,7 @@
 //  order_levels : the level slots by falling window length (counting sort of
 //                 the window kernel's buckets), so that the queues below hand
 //                 out the longest work first;
-//  levels<NW>   : a group takes a level from a device queue and carries it
+//  levels       : a group takes a level from a device queue and carries it
 //                 through
 //                   1. FP32 passes: safeguarded Cooley-Newton with the count
 //                      bracket, to a Newton step of at most kTol32;
@@ -17,14 +17,15 @@
 //                      as tagged float pairs, then turned into the normalised
 //                      doubles and the row's rest zeroed while the window is
 //                      still in the caches.
-//                 NW = 1 (a warp) where there are levels enough to fill the
-//                 GPU, NW = 8 (a CTA) for windows above a threshold that falls
-//                 with the number of levels;
+//                 The group is a warp where there are levels enough to fill
+//                 the GPU, a CTA for windows above a threshold that falls with
+//                 the number of levels, a cluster of four CTAs for the longest
+//                 windows of a few potentials;
 //  repair       : levels stage 2 could not settle (full double-float passes
 //                 from the scan bracket widened by one trial spacing) and
 //                 levels whose final pass disagrees (twist-index search), one
 //                 CTA per level;
-//  rewrite<NW>  : psi again from the final energies and match points (the
+//  rewrite      : psi again from the final energies and match points (the
 //                 adjoint of a solve that kept none), the same passes as the
 //                 solve's, so the same bits.
 #include <cuda_runtime.h>
@@ -42,15 +43,9 @@ namespace epscu {
 
 namespace {
 
-constexpr int kWarpThreads = 128;  // four one-warp groups in a CTA
-constexpr int kWarpCtasPerSm = 4;
 constexpr int kCtaWarps = 8;
+constexpr int kClusterWarps = 32;  // four CTAs
 constexpr int kCtaCtasPerSm = 2;
-
-template <int NW>
-constexpr int cta_threads() { return NW == 1 ? kWarpThreads : 32 * NW; }
-template <int NW>
-constexpr int ctas_per_sm() { return NW == 1 ? kWarpCtasPerSm : kCtaCtasPerSm; }
 
 // FP32 Newton steps at most this large hand over to the double-float passes
 // (Hartree); the energy after such a step is far inside their first step's
@@ -153,19 +148,19 @@ __device__ __noinline__ PassDF norm_pass(const Grp<NW> G, const Chunk& c, const 
         So = dfe_to_double(so);
         Si = dfe_to_double(si);
     } else {
-        if (t == c.Lo - 1) sh.eo3 = s;
-        if (t == c.Lo + c.Li - 1) sh.ei3 = s;
+        if (t == c.Lo - 1) G.put(sh.eo3, s);
+        if (t == c.Lo + c.Li - 1) G.put(sh.ei3, s);
         if (lane == 0) {
             const int w = G.warp();
-            sh.nodes3[w] = nodes;
-            sh.so[w] = so;
-            sh.si[w] = si;
-            sh.po_L[w] = po_L;
-            sh.po_i[w] = po_i;
-            sh.pi_L[w] = pi_L;
-            sh.pi_i[w] = pi_i;
+            G.put(sh.nodes3[w], nodes);
+            G.put(sh.so[w], so);
+            G.put(sh.si[w], si);
+            G.put(sh.po_L[w], po_L);
+            G.put(sh.po_i[w], po_i);
+            G.put(sh.pi_L[w], pi_L);
+            G.put(sh.pi_i[w], pi_i);
         }
-        __syncthreads();
+        G.sync();
         Eo = sh.eo3;
         Ei = sh.ei3;
         nodes = 0;
@@ -213,10 +208,10 @@ __device__ __noinline__ PassDF norm_pass(const Grp<NW> G, const Chunk& c, const 
         r.dE = r.gamma * fk * fk / (12.0 * a * r.sum);
     }
     if constexpr (NW > 1) {
-        if (t == 0) sh.res = r;
-        __syncthreads();
+        if (t == 0) G.put(sh.res, r);
+        G.sync();
         r = sh.res;
-        __syncthreads();  // every thread has the result before the next pass's
+        G.sync();  // every thread has the result before the next pass's
     }
     return r;
 }
@@ -292,13 +287,13 @@ struct States {
         }
         if constexpr (NW > 1) {
             if (G.leader()) {
-                sh.res.dE = dE;
-                sh.res.count = count;
+                G.put(sh.res.dE, dE);
+                G.put(sh.res.count, count);
             }
-            __syncthreads();
+            G.sync();
             dE = sh.res.dE;
             count = sh.res.count;
-            __syncthreads();
+            G.sync();
         }
         return dE;
     }
@@ -373,10 +368,10 @@ __device__ __forceinline__ void norm_level(const Grp<NW>& G, const DevBatch& b, 
     w.E = E;
     if (NW == 1 || G.warp() == 0) finalize_df(b.meta[w.p], w, best, k);
     if constexpr (NW > 1) {
-        if (G.leader()) sh.w = w;
-        __syncthreads();
+        if (G.leader()) G.put(sh.w, w);
+        G.sync();
         w = sh.w;
-        __syncthreads();
+        G.sync();
     }
 }
 
@@ -474,7 +469,7 @@ __global__ void __launch_bounds__(kLists * kBuckets) order_levels_kernel(DevBatc
     static_assert(kBuckets == 64, "two warps scan a list's buckets");
     __shared__ int s_first[kLists * kBuckets];
     __shared__ int s_half[kLists];
-    int32_t* const lists[kLists] = {b.warp_list, b.long_list, b.fragile_list, b.fragile_long};
+    int32_t* const lists[kLists] = {b.warp_list, b.long_list, b.fragile_list, b.fragile_long, b.cluster_list};
     {
         // exclusive sums over falling bucket number, each list by two warps
         const int list = threadIdx.x / kBuckets, q = threadIdx.x % kBuckets;
@@ -490,7 +485,8 @@ __global__ void __launch_bounds__(kLists * kBuckets) order_levels_kernel(DevBatc
         if (q >= 32) x += s_half[list];
         s_first[bucket] = x - n;
         if (blockIdx.x == 0 && q == kBuckets - 1) {
-            int32_t* const count[kLists] = {&b.hdr->n_warp, &b.hdr->n_long, &b.hdr->n_fragile, &b.hdr->n_fragile_long};
+            int32_t* const count[kLists] = {&b.hdr->n_warp, &b.hdr->n_long, &b.hdr->n_fragile, &b.hdr->n_fragile_long,
+                                            &b.hdr->n_cluster};
             *count[list] = x;
         }
         __syncthreads();
@@ -502,14 +498,23 @@ __global__ void __launch_bounds__(kLists * kBuckets) order_levels_kernel(DevBatc
     }
 }
 
+// The lists of the groups of NW warps
 template <int NW>
-__global__ void __launch_bounds__(cta_threads<NW>(), ctas_per_sm<NW>()) levels_kernel(DevBatch b) {
-    __shared__ SharedDF<NW> sh;  // (a one-warp group uses neither)
-    __shared__ Shared32<NW> sh32;
+__device__ __forceinline__ const int32_t* level_list(const DevBatch& b) {
+    return NW == 1 ? b.warp_list : NW == kCtaWarps ? b.long_list : b.cluster_list;
+}
+template <int NW>
+__device__ __forceinline__ int level_count(const DevBatch& b) {
+    return min(NW == 1 ? b.hdr->n_warp : NW == kCtaWarps ? b.hdr->n_long : b.hdr->n_cluster, b.max_levels);
+}
+
+// The levels of one list, until its queue is empty.
+template <int NW>
+__device__ __forceinline__ void level_queue(const DevBatch& b, SharedDF<NW>& sh, Shared32<NW>& sh32) {
     const Grp<NW> G;
-    const int32_t* list = NW == 1 ? b.warp_list : b.long_list;
-    const int n = min(NW == 1 ? b.hdr->n_warp : b.hdr->n_long, b.max_levels);
-    int32_t* queue = &b.hdr->queue[NW == 1 ? kQWarpLevels : kQLongLevels];
+    const int32_t* list = level_list<NW>(b);
+    const int n = level_count<NW>(b);
+    int32_t* queue = &b.hdr->queue[NW == 1 ? kQWarpLevels : NW == kCtaWarps ? kQLongLevels : kQClusterLevels];
     Tally tally;
     for (;;) {
         const int2 next = grp_take<NW>(G, b, queue, n, sh.word);
@@ -632,6 +637,33 @@ __global__ void __launch_bounds__(cta_threads<NW>(), ctas_per_sm<NW>()) levels_k
     if (G.leader()) flush(b, tally, NW > 1);
 }
 
+// The levels of all lists, the longest windows first: a CTA per level while
+// there are long ones, then its warps a level each (one kernel: the warp list's
+// longest marches run beside the last of the CTA list's instead of after them;
+// 56 levels of one 4096-point grid 160 -> 85 us, 64 x 57 levels 670 -> 525 us).
+__global__ void __launch_bounds__(32 * kCtaWarps, kCtaCtasPerSm) levels_kernel(DevBatch b) {
+    __shared__ SharedDF<kCtaWarps> sh;
+    __shared__ Shared32<kCtaWarps> sh32;
+    __shared__ SharedDF<1> sh1;  // (a one-warp group uses neither)
+    __shared__ Shared32<1> sh321;
+    level_queue<kCtaWarps>(b, sh, sh32);
+    level_queue<1>(b, sh1, sh321);
+}
+
+__global__ void __cluster_dims__(kClusterWarps / kCtaWarps, 1, 1)
+    __launch_bounds__(32 * kCtaWarps, kCtaCtasPerSm) cluster_levels_kernel(DevBatch b) {
+    __shared__ SharedDF<kClusterWarps> sh;
+    __shared__ Shared32<kClusterWarps> sh32;
+    Grp<kClusterWarps>().sync();  // (the other CTAs' shared memory exists)
+    __shared__ SharedDF<kCtaWarps> sh8;
+    __shared__ Shared32<kCtaWarps> sh328;
+    __shared__ SharedDF<1> sh1;
+    __shared__ Shared32<1> sh321;
+    level_queue<kClusterWarps>(b, sh, sh32);
+    level_queue<kCtaWarps>(b, sh8, sh328);
+    level_queue<1>(b, sh1, sh321);
+}
+
 // Levels the queues above left over: first those stage 2 could not settle
 // (the FP32 bracket may be off by its count errors: safeguarded Cooley-Newton
 // with double-float passes from the FP32 stage's bracket, or the scan's widened
@@ -743,10 +775,10 @@ __global__ void __launch_bounds__(32 * kCtaWarps, kCtaCtasPerSm) repair_kernel(D
         if (row) finish_row<Grp<NW>::kThreads>(G.t(), w, row, L.N);
         if (G.leader()) {
             w.iters += ndf;
-            if (!(w.status & EPSCU_STATUS_LONG)) {
+            if ((w.status & (EPSCU_STATUS_LONG | EPSCU_STATUS_CLUSTER)) != EPSCU_STATUS_LONG) {
                 const int at = atomicAdd(&b.hdr->n_long, 1);
                 if (at < b.max_levels) b.long_list[at] = slot;
-                w.status |= EPSCU_STATUS_LONG;
+                w.status = (w.status & ~EPSCU_STATUS_CLUSTER) | EPSCU_STATUS_LONG;
             }
             b.levels[slot] = w;
         }
@@ -757,17 +789,19 @@ __global__ void __launch_bounds__(32 * kCtaWarps, kCtaCtasPerSm) repair_kernel(D
 
 // psi of the listed levels from their final energies and match points.
 template <int NW>
-__global__ void __launch_bounds__(cta_threads<NW>(), ctas_per_sm<NW>()) rewrite_kernel(DevBatch b) {
-    __shared__ SharedDF<NW> sh;
+__device__ __forceinline__ void rewrite_queue(const DevBatch& b, SharedDF<NW>& sh) {
     const Grp<NW> G;
     if (!b.psi || b.hdr->error) return;
-    const int32_t* list = NW == 1 ? b.warp_list : b.long_list;
-    const int n = min(NW == 1 ? b.hdr->n_warp : b.hdr->n_long, b.max_levels);
+    const int32_t* list = level_list<NW>(b);
+    const int n = level_count<NW>(b);
+    int32_t* queue = &b.hdr->queue[NW == 1 ? kQWarpRewrite : NW == kCtaWarps ? kQLongRewrite : kQClusterRewrite];
     for (;;) {
-        const int2 next = grp_take<NW>(G, b, &b.hdr->queue[NW == 1 ? kQWarpRewrite : kQLongRewrite], n, sh.word);
+        const int2 next = grp_take<NW>(G, b, queue, n, sh.word);
         if (next.x >= n) break;
         LevelWork w = b.levels[list[next.x]];
-        if (NW == 1 && (w.status & EPSCU_STATUS_LONG)) continue;  // (a repaired level: on the long list too)
+        // (a repaired level: on the long list too)
+        if (NW == 1 && (w.status & EPSCU_STATUS_LONG)) continue;
+        if (NW == kClusterWarps && !(w.status & EPSCU_STATUS_CLUSTER)) continue;
         const Level L = level_of(b, w);
         double* row = b.psi + b.meta[w.p].psi_off + (int64_t)(w.v - b.min_level) * L.N;
         if (!no_result(w)) {
@@ -780,37 +814,62 @@ __global__ void __launch_bounds__(cta_threads<NW>(), ctas_per_sm<NW>()) rewrite_
     }
 }
 
+__global__ void __launch_bounds__(32 * kCtaWarps, kCtaCtasPerSm) rewrite_kernel(DevBatch b) {
+    __shared__ SharedDF<kCtaWarps> sh;
+    __shared__ SharedDF<1> sh1;
+    rewrite_queue<kCtaWarps>(b, sh);
+    rewrite_queue<1>(b, sh1);
+}
+
+__global__ void __cluster_dims__(kClusterWarps / kCtaWarps, 1, 1)
+    __launch_bounds__(32 * kCtaWarps, kCtaCtasPerSm) cluster_rewrite_kernel(DevBatch b) {
+    __shared__ SharedDF<kClusterWarps> sh;
+    Grp<kClusterWarps>().sync();
+    __shared__ SharedDF<kCtaWarps> sh8;
+    __shared__ SharedDF<1> sh1;
+    rewrite_queue<kClusterWarps>(b, sh);
+    rewrite_queue<kCtaWarps>(b, sh8);
+    rewrite_queue<1>(b, sh1);
+}
+
 }  // namespace
 
 namespace {
 
 // the staging buffers of a CTA's warps, as dynamic shared memory
 constexpr size_t stage_bytes(int threads) { return (size_t)(threads / 32) * kStageFloat2 * sizeof(float2); }
-constexpr size_t kWarpStage = stage_bytes(kWarpThreads), kCtaStage = stage_bytes(32 * kCtaWarps);
+constexpr size_t kCtaStage = stage_bytes(32 * kCtaWarps);
 
 }  // namespace
 
 void levels_set_attributes() {
-    cudaFuncSetAttribute(levels_kernel<kCtaWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtaStage);
-    cudaFuncSetAttribute(rewrite_kernel<kCtaWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtaStage);
-    cudaFuncSetAttribute(repair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtaStage);
+    const auto stage = [](const void* f) {
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCtaStage);
+    };
+    stage((const void*)levels_kernel);
+    stage((const void*)cluster_levels_kernel);
+    stage((const void*)rewrite_kernel);
+    stage((const void*)cluster_rewrite_kernel);
+    stage((const void*)repair_kernel);
 }
 
 void launch_order_levels(const DevBatch& b, int sm_count, cudaStream_t s) {
     order_levels_kernel<<<sm_count, kLists * kBuckets, 0, s>>>(b);
 }
-void launch_warp_levels(const DevBatch& b, int sm_count, cudaStream_t s) {
-    levels_kernel<1><<<sm_count * kWarpCtasPerSm, kWarpThreads, kWarpStage, s>>>(b);
-}
-void launch_long_levels(const DevBatch& b, int sm_count, cudaStream_t s) {
-    levels_kernel<kCtaWarps><<<sm_count * kCtaCtasPerSm, 32 * kCtaWarps, kCtaStage, s>>>(b);
+void launch_levels(const DevBatch& b, int sm_count, cudaStream_t s) {
+    if (b.cluster_list)
+        cluster_levels_kernel<<<sm_count / 4 * 4 * kCtaCtasPerSm, 32 * kCtaWarps, kCtaStage, s>>>(b);
+    else
+        levels_kernel<<<sm_count * kCtaCtasPerSm, 32 * kCtaWarps, kCtaStage, s>>>(b);
 }
 void launch_repair(const DevBatch& b, int sm_count, cudaStream_t s) {
     repair_kernel<<<sm_count * kCtaCtasPerSm, 32 * kCtaWarps, kCtaStage, s>>>(b);
 }
 void launch_rewrite(const DevBatch& b, int sm_count, cudaStream_t s) {
-    rewrite_kernel<kCtaWarps><<<sm_count * kCtaCtasPerSm, 32 * kCtaWarps, kCtaStage, s>>>(b);
-    rewrite_kernel<1><<<sm_count * kWarpCtasPerSm, kWarpThreads, kWarpStage, s>>>(b);
+    if (b.cluster_list)
+        cluster_rewrite_kernel<<<sm_count / 4 * 4 * kCtaCtasPerSm, 32 * kCtaWarps, kCtaStage, s>>>(b);
+    else
+        rewrite_kernel<<<sm_count * kCtaCtasPerSm, 32 * kCtaWarps, kCtaStage, s>>>(b);
 }
 
 }  // namespace epscu

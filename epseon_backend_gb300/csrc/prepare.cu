@@ -772,6 +772,8 @@ __global__ void __launch_bounds__(128) window_kernel(DevBatch b) {
     const int n_warps = (gridDim.x * blockDim.x) >> 5;
     const int total = b.hdr->total_levels;
     const int long_min = b.long_window > 0 ? b.long_window : default_long_window(total);
+    const int cluster_min =
+        b.cluster_list && b.long_window < kMinClusterWindow ? default_cluster_window(total) : 0x7fffffff;
     const int fragile_min = b.long_window > 0 ? b.long_window : default_fragile_window(total);
     for (int slot = warp; slot < total; slot += n_warps) {
         const LevelWork w = b.levels[slot];
@@ -787,7 +789,7 @@ __global__ void __launch_bounds__(128) window_kernel(DevBatch b) {
                                  w.n_in_bracket > 1 || (s > 0 && w.hi0 - b.levels[slot - 1].lo0 < kFragileGap) ||
                                  (s + 1 < m.n_out && b.levels[slot + 1].hi0 - w.lo0 < kFragileGap);
             list = fragile ? (len > fragile_min ? kListFragileLong : kListFragile)
-                           : (len > long_min ? kListLong : kListWarp);
+                           : (len > cluster_min ? kListCluster : len > long_min ? kListLong : kListWarp);
         }
         if ((threadIdx.x & 31) == 0) {
             const int bucket = list * kBuckets + length_bucket(len);
@@ -798,6 +800,7 @@ __global__ void __launch_bounds__(128) window_kernel(DevBatch b) {
             out->bucket = bucket;
             out->rank = atomicAdd(&b.hdr->hist[bucket], 1);
             if (list == kListLong || list == kListFragileLong) out->status = w.status | EPSCU_STATUS_LONG;
+            if (list == kListCluster) out->status = w.status | EPSCU_STATUS_LONG | EPSCU_STATUS_CLUSTER;
         }
     }
 }

@@ -12,6 +12,18 @@ namespace epscu {
 
 namespace {
 
+// the barrier of a group of NT threads: a warp, the CTA, a cluster of CTAs of 256
+template <int NT>
+__device__ __forceinline__ void group_sync() {
+    if constexpr (NT == 32) __syncwarp();
+    else if constexpr (NT <= 256) __syncthreads();
+    else
+        asm volatile(
+            "barrier.cluster.arrive.release;\n\t"
+            "barrier.cluster.wait.acquire;" ::
+                : "memory");
+}
+
 // n zeros at p by NT threads (t: this one), 16 bytes a store
 template <int NT>
 __device__ __forceinline__ void zero_points(int t, double* p, int n) {
@@ -40,8 +52,7 @@ __device__ __noinline__ void finish_row(int t, const LevelWork& w, double* __res
     e_out -= w.ex_out;
     e_in -= w.ex_in;
     // the pairs were stored by other threads of the group
-    if constexpr (NT == 32) __syncwarp();
-    else __syncthreads();
+    group_sync<NT>();
     const float2* pair = reinterpret_cast<const float2*>(row);
     constexpr int kS = NT;
     for (int i0 = w.j0; i0 <= w.j1; i0 += 4 * kS) {
