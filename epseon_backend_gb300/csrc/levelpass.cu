@@ -51,6 +51,9 @@ constexpr int kCtaCtasPerSm = 2;
 // (Hartree); the energy after such a step is far inside their first step's
 // range
 constexpr double kTol32 = 3e-8;
+// halvings before the repair kernel looks for a better match point (256 bumped
+// Morse wells: the kernel 1.0 ms without, 0.51 ms after 4, 0.39 ms after 2)
+constexpr int kHalveFirst = 2;
 
 // match points on a strip boundary (whole strips on the outward side) where
 // the window allows it
@@ -714,12 +717,13 @@ __global__ void __launch_bounds__(32 * kCtaWarps, kCtaCtasPerSm) repair_kernel(D
                 hi = fmin(m.e_cap, w.hi0 + m.delta);
             }
             if (!(E > lo && E < hi)) E = 0.5 * (lo + hi);
-            bool moved = false, done = false;
+            bool moved = false, done = false, twisted = false;
+            int halved = 0;
             for (int it = 0, cap = fallback_cap(b); it < cap; ++it) {
                 // sum psi^2 and the peak in FP32, the state and count in
                 // double-float
                 const Pass32 f = pass32<NW, true>(G, L.Wf, df_from_double(__dmul_rn(L.a, E)), L.j0, L.j1, k, L.steep, sh32);
-                if (f.peak_log2 >= 2 && !moved) {
+                if (f.peak_log2 >= 2 && !moved && !twisted) {
                     const int kp = align_k(L.j0, L.j1, f.peak_i);
                     moved = true;
                     if (kp != k) {
@@ -743,6 +747,15 @@ __global__ void __launch_bounds__(32 * kCtaWarps, kCtaCtasPerSm) repair_kernel(D
                     }
                 } else {
                     E = 0.5 * (lo + hi);
+                    // (matched in the wrong well the pass never has the level's
+                    // nodes, and halving the bracket to the energy's resolution
+                    // takes ~25 passes more: look for a better point instead)
+                    twisted = b.twist_list && (++halved == kHalveFirst || halved == 2 * kHalveFirst);
+                    if (twisted) {
+                        k = twist_point<NW>(G, L, E, b.twist_scratch + (int64_t)blockIdx.x * b.twist_stride,
+                                            b.twist_stride, k, sh);
+                        ndf += 2;
+                    }
                 }
                 if (hi - lo <= tol) {
                     E = 0.5 * (lo + hi);
