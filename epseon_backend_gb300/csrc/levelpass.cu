@@ -73,8 +73,8 @@ __device__ __forceinline__ dfl df_neg(dfl a) { return {-a.h, -a.l}; }
 // unnormalised psi-hat of every window point as tagged pairs.
 template <int NW>
 __device__ __noinline__ PassDF norm_pass(const Grp<NW> G, const Chunk& c, const float2* __restrict__ Wf, double a,
-                                            double Wk, double E, int k, const StD& X, double* __restrict__ row,
-                                            SharedDF<NW>& sh) {
+                                            double Wk, double E, int k, const StD& X, bool neg,
+                                            double* __restrict__ row, SharedDF<NW>& sh) {
     constexpr unsigned full = 0xffffffffu;
     const int t = G.t(), lane = G.lane();
     const dfl aE = df_from_double(__dmul_rn(a, E));
@@ -82,7 +82,7 @@ __device__ __noinline__ PassDF norm_pass(const Grp<NW> G, const Chunk& c, const 
     PsiTag tag = psi_tag(s.e);
     SqSum ss;
     ss.init();
-    int nodes = 0, last = 0;
+    int nodes = 0, last = 0, flip = 0;
     int pk_L = -(1 << 30), pk_i = k;
     for_points(
         c, Wf, [&](float2 w) { return df_point(aE, w); },
@@ -94,7 +94,8 @@ __device__ __noinline__ PassDF norm_pass(const Grp<NW> G, const Chunk& c, const 
             if (row) slot[i & (kStrip - 1)] = psi_pair(psi, tag);
             const float before = s.u.h;
             df_march(pt.q, s.u, s.d);
-            nodes += (__float_as_uint(s.u.h) ^ __float_as_uint(before)) >> 31;
+            flip = (int)((__float_as_uint(s.u.h) ^ __float_as_uint(before)) >> 31);
+            nodes += flip;
             last = i;
         },
         [&]() {
@@ -133,6 +134,12 @@ __device__ __noinline__ PassDF norm_pass(const Grp<NW> G, const Chunk& c, const 
             }
         });
     const bool out = t < c.Lo;
+    // A zero of psi on a chunk's end point (the centre of a symmetric well): the
+    // march gives u there one sign, the next thread's start state may have the
+    // other, and the change would be counted by both threads or by neither.
+    // The start state's sign holds.
+    if (c.ns > 0 && t != c.Lo - 1 && t != c.Lo + c.Li - 1 && neg != ((__float_as_uint(s.u.h) >> 31) != 0))
+        nodes += flip ? -1 : 1;
     nodes = __reduce_add_sync(full, nodes);
     const DfE mine = c.ns > 0 ? sqsum_dfe(ss, 2 * s.e) : DfE{{0.0f, 0.0f}, 0};
     DfE so = warp_sum_dfe(out ? mine : DfE{{0.0f, 0.0f}, 0});
@@ -269,10 +276,11 @@ struct States {
     Chunk c;
     StD X, Eo, Ei;
     int nodes;
+    bool neg;
 
     __device__ __forceinline__ void run(const Grp<NW>& G, const Level& L, double E, int k, SharedDF<NW>& sh) {
         c = make_chunk(G.t(), Grp<NW>::kThreads, L.j0, L.j1, k, L.steep);
-        states_df<NW>(G, c, L.Wf, df_from_double(__dmul_rn(L.a, E)), sh, X, Eo, Ei, nodes);
+        states_df<NW>(G, c, L.Wf, df_from_double(__dmul_rn(L.a, E)), sh, X, Eo, Ei, nodes, neg);
     }
 
     // run() and the Cooley correction at its match point, with the sum of an
@@ -319,7 +327,7 @@ __device__ __forceinline__ void norm_level(const Grp<NW>& G, const DevBatch& b, 
         }
         have = false;
         ++n_pass;
-        return norm_pass<NW>(G, st.c, L.Wf, L.a, __ldg(L.W + kk), E, kk, st.X, row, sh);
+        return norm_pass<NW>(G, st.c, L.Wf, L.a, __ldg(L.W + kk), E, kk, st.X, st.neg, row, sh);
     };
     PassDF r, best;
     int kk = k, k_row = k;
@@ -409,7 +417,8 @@ __device__ __forceinline__ int twist_point(const Grp<NW>& G, const Level& L, dou
         c.seg = c.ns > 0 ? 0 : G.t();
         StD X, Eo, Ei;
         int nodes;
-        states_df<NW>(G, c, L.Wf, aE, sh, X, Eo, Ei, nodes);
+        bool neg;
+        states_df<NW>(G, c, L.Wf, aE, sh, X, Eo, Ei, nodes, neg);
         dfl u = X.u, d = X.d;
         for_points(
             c, L.Wf, [&](float2 w) { return df_point(aE, w); },
@@ -421,7 +430,11 @@ __device__ __forceinline__ int twist_point(const Grp<NW>& G, const Level& L, dou
                         rho[rel / kTwistSample] = ratio;
                     } else if (i <= L.j1 - 1) {
                         const double Ti = aEd - __ldg(L.W + i);
-                        const double gam = fabs(-12.0 * Ti / (1.0 + Ti) + rho[rel / kTwistSample] + ratio);
+                        const double out = rho[rel / kTwistSample];
+                        // (with the rounding of the two ratios: at a node of psi they are huge
+                        // and may cancel to anything)
+                        const double gam =
+                            fabs(-12.0 * Ti / (1.0 + Ti) + out + ratio) + 0x1p-44 * (fabs(out) + fabs(ratio));
                         if (gam < best || (gam == best && i < at)) {
                             best = gam;
                             at = i;
@@ -776,7 +789,7 @@ __global__ void __launch_bounds__(32 * kCtaWarps, kCtaCtasPerSm) repair_kernel(D
 #pragma unroll 1
             for (int it = 0;; ++it) {
                 st.run(G, L, E, k, sh);
-                r = norm_pass<NW>(G, st.c, L.Wf, L.a, __ldg(L.W + k), E, k, st.X, row, sh);
+                r = norm_pass<NW>(G, st.c, L.Wf, L.a, __ldg(L.W + k), E, k, st.X, st.neg, row, sh);
                 ndf += 2;
                 if (it >= 8 || r.nodes != w.v || !isfinite(r.dE) || !(fabs(r.dE) < 1e-7)) break;
                 if (fabs(r.dE) <= 1e-13 * fmax(1.0, fabs(E))) break;
@@ -820,7 +833,7 @@ __device__ __forceinline__ void rewrite_queue(const DevBatch& b, SharedDF<NW>& s
         if (!no_result(w)) {
             States<NW> st;
             st.run(G, L, w.E, w.k, sh);
-            const PassDF r = norm_pass<NW>(G, st.c, L.Wf, L.a, __ldg(L.W + w.k), w.E, w.k, st.X, row, sh);
+            const PassDF r = norm_pass<NW>(G, st.c, L.Wf, L.a, __ldg(L.W + w.k), w.E, w.k, st.X, st.neg, row, sh);
             finalize_df(b.meta[w.p], w, r, w.k);
         }
         finish_row<Grp<NW>::kThreads>(G.t(), w, row, L.N);
