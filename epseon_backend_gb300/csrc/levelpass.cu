@@ -85,7 +85,7 @@ __device__ __noinline__ PassDF norm_pass(const Grp<NW> G, const Chunk& c, const 
     int nodes = 0, last = 0, flip = 0;
     int pk_L = -(1 << 30), pk_i = k;
     for_points(
-        c, Wf, [&](float2 w) { return df_point(aE, w); },
+        c, Wf, [&](float2 w) { return df_point<true>(aE, w, c.steep); },
         [&](const PointDF& pt, float2* slot, int i) {
             const dfl psi = df_mul(s.u, pt.r);
             const float p = __fmul_rn(psi.h, psi.h);
@@ -421,7 +421,7 @@ __device__ __forceinline__ int twist_point(const Grp<NW>& G, const Level& L, dou
         states_df<NW>(G, c, L.Wf, aE, sh, X, Eo, Ei, nodes, neg);
         dfl u = X.u, d = X.d;
         for_points(
-            c, L.Wf, [&](float2 w) { return df_point(aE, w); },
+            c, L.Wf, [&](float2 w) { return df_point<false>(aE, w, c.steep); },
             [&](const PointDF& pt, float2*, int i) {
                 const int rel = i - L.j0;
                 if (rel % kTwistSample == 0 && rel / kTwistSample < stride) {
