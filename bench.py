@@ -4,8 +4,8 @@ N ~ logU[2048, 65536], 8192 trial energies, levels up to 0.999 De), counting
 only levels within 1e-9 Hartree of the FP64 reference and with the right
 node count.
 
-One step = one device-resident solve (FP32 TMA scan, FP32 Cooley refinement,
-FP64 polish, normalised psi written to HBM, replayed from a CUDA graph) plus
+One step = one device-resident solve (FP32 scan, FP32 and double-float Cooley
+passes, normalised psi written to HBM, replayed from a CUDA graph) plus
 the Hellmann-Feynman adjoint of L = sum_v w_v (E_v - T_v)^2 back to every
 V(r_i).  The plain FP64 CUDA solver (FP64 scan + FP64 bisection + psi) is timed
 on the same batch and is also the per-level FP64 reference (it is bit-exact
@@ -42,10 +42,10 @@ CPU_SAMPLE = 96  # potentials of the workload the CPU legs time
 # dram__bytes_read.sum + dram__bytes_write.sum of one scan32 launch per grid
 # point, ncu on the 128-potential mixed batch (18.12 MB / 2,242,300 points)
 SCAN32_DRAM_BYTES_PER_POINT = 8.08
-# ncu (dram__bytes_read.sum + dram__bytes_write.sum) of refine_long_kernel per
-# algorithmic point-update on the 512-potential mixed batch (64.05 MB over
-# 235,987,411 point-updates: the windows' W is re-read from L2)
-REFINE_LONG_DRAM_BYTES_PER_UPDATE = 0.2714
+# ncu (dram__bytes_read.sum + dram__bytes_write.sum) of levels_kernel per
+# point-update on the 512-potential mixed batch (5.18 GB, the psi rows and the
+# windows' W, over 452,052,088 point-updates)
+LEVELS_DRAM_BYTES_PER_UPDATE = 11.5
 
 
 def dist_env():
@@ -431,38 +431,39 @@ def main():
                "sample": f"{len(idx)} of {len(b)} potentials (seeded random), plain FP64 method, {dt:.1f} s",
                "plain_gpu_bit_exact_on_sample": bool(same)}
 
-    # ---- roofline of the dominant kernel: refine_long_kernel, the longest
-    # single launch of the step (the long levels' CTA-per-level refinement;
-    # time from its own events in the stage-timed solve, on the solve stream).
-    # Unit: one Numerov point-update = 9 algorithmic flops (T, f, g, two-term
-    # recurrence) in its FP32 and its double-float passes alike; the chunked
-    # three-phase passes, the compensation (a double-float step issues ~10x
-    # the FP32 instructions), renormalisation and sign bookkeeping are not
-    # counted, so the fraction is structurally far below 1.
-    rl_updates = int(st.long_fp32_point_updates + st.long_df_point_updates)
-    ach = 9.0 * rl_updates / (st.ms_refine_long * 1e-3) / 1e12 if st.ms_refine_long > 0 else 0.0
-    traffic = (REFINE_LONG_DRAM_BYTES_PER_UPDATE * rl_updates) if REFINE_LONG_DRAM_BYTES_PER_UPDATE else None
+    # ---- roofline of the dominant kernel: levels_kernel, which carries the
+    # levels from the scan's bracket to the psi rows, with the fragile levels'
+    # kernel and the two repair kernels (the level stages of the stage-timed
+    # solve, which share one count of point-updates).  Unit: one Numerov
+    # point-update = 9 algorithmic flops (T, f, g, two-term recurrence) in its
+    # FP32 and its double-float passes alike; the second column of the transfer
+    # matrices, the compensation (a double-float step issues ~3x the FP32
+    # instructions), renormalisation and sign bookkeeping are not counted, so
+    # the fraction is structurally far below 1.
+    rl_updates = int(st.refine_point_updates + st.fp64_point_updates)
+    level_ms = st.ms_refine32 + st.ms_polish64
+    ach = 9.0 * rl_updates / (level_ms * 1e-3) / 1e12 if level_ms > 0 else 0.0
     roof = {"bound": "fp32_alu", "achieved": ach, "peak": fp32_peak, "unit": "TFLOP/s", "frac": ach / fp32_peak,
-            "traffic": traffic,
-            "traffic_unit": "bytes per launch (ncu-measured DRAM bytes per point-update x point-updates)",
-            "kernel": "refine_long_kernel", "ms": st.ms_refine_long,
-            "algorithmic": {"point_updates": rl_updates, "fp32_pass_point_updates": int(st.long_fp32_point_updates),
-                            "double_float_pass_point_updates": int(st.long_df_point_updates),
+            "traffic": LEVELS_DRAM_BYTES_PER_UPDATE * rl_updates,
+            "traffic_unit": "bytes per step (ncu-measured DRAM bytes per point-update x point-updates, psi rows included)",
+            "kernel": "levels_kernel (+ repair_kernel, fragile_kernel, fragile_repair_kernel)", "ms": level_ms,
+            "levels_kernel_ms": st.ms_refine_long,
+            "algorithmic": {"point_updates": rl_updates, "fp32_pass_point_updates": int(st.refine_point_updates),
+                            "double_float_pass_point_updates": int(st.fp64_point_updates),
                             "flops_per_update": 9},
             "peak_source": "measured FP32 FMA burst (epscu_measure_fma_peaks), 2 flops per FMA"}
-    # the scan stage in the same unit (the coarse scan32 launch plus, on large
-    # batches, the bisection rounds; scan32 alone is FP32-issue-bound)
+    # the scan stage in the same unit (large batches: the coarse scan32 launch
+    # and the bisection round; smaller ones: the group counts)
     scan_ach = 9.0 * st.scan_point_updates / (st.ms_scan * 1e-3) / 1e12
-    roof_scan = {"kernel": "scan stage (scan32_kernel" + (" on every 16th trial energy + the bisection count round)"
-                                                          if len(b) >= 512 else ")"),
+    roof_scan = {"kernel": "scan stage (" + ("scan32_kernel on every 16th trial energy + the bisection count round)"
+                                             if len(b) >= 512 else "count_stride_kernel, count_listed_kernel)"),
                  "achieved": scan_ach, "peak": fp32_peak, "unit": "TFLOP/s", "frac": scan_ach / fp32_peak,
                  "ms": st.ms_scan, "point_updates": int(st.scan_point_updates),
                  "dram_bytes_per_grid_point_scan32": SCAN32_DRAM_BYTES_PER_POINT}
-    # the per-level stages in the same unit (algorithmic point-updates counted
-    # by the kernels over the level windows; latency-bound lane marches)
+    # point-updates of the level stages (counted by the kernels over the level
+    # windows) per second of those stages
     stage_rates = {
-        "refine32_point_updates_per_s": st.refine_point_updates / (st.ms_refine32 * 1e-3) if st.ms_refine32 > 0 else None,
-        "double_float_point_updates_per_s": st.fp64_point_updates / (st.ms_polish64 * 1e-3) if st.ms_polish64 > 0 else None,
+        "level_point_updates_per_s": rl_updates / (level_ms * 1e-3) if level_ms > 0 else None,
         "refine32_point_updates": int(st.refine_point_updates),
         "double_float_point_updates": int(st.fp64_point_updates),
     }
@@ -472,25 +473,17 @@ def main():
     roof_plain["frac"] = roof_plain["achieved"] / fp64_peak
     peaks = measured_peaks()
     hbm = peaks.get("hbm_gbs")
-    # the psi write-back, kernel by kernel (stage-timed solve): zero_psi
-    # writes the zeros outside the level windows (8 B a point), the norm
-    # passes store each window point once as a tagged float pair (8 B, inside
-    # their compute-bound passes, not timed here), scale_psi reads the pairs
-    # and writes the normalised doubles (16 B a window point).  Algorithmic
-    # bytes: the rows written once, levels x N x 8 B.
+    # the psi write-back, inside the level kernels: zeros outside the level
+    # windows (8 B a point), the window points stored once as tagged float
+    # pairs (8 B), read back from the caches and written as the normalised
+    # doubles (16 B).  Algorithmic bytes: the rows written once, levels x N x 8 B.
     zero_bytes = 8 * int(st.psi_zero_points)
-    scale_bytes = 16 * int(st.psi_window_points)
-    pair_bytes = 8 * int(st.psi_window_points)
-
-    def gbs(nbytes, ms_):
-        return nbytes / (ms_ * 1e-3) / 1e9 if ms_ > 0 else None
-
+    window_bytes = 24 * int(st.psi_window_points)
     psi_write = {
         "algorithmic_bytes": int(st.psi_bytes),
-        "zero_psi": {"bytes": zero_bytes, "ms": st.ms_zero_psi, "GB_per_s": gbs(zero_bytes, st.ms_zero_psi)},
-        "scale_psi": {"bytes": scale_bytes, "ms": st.ms_write, "GB_per_s": gbs(scale_bytes, st.ms_write)},
-        "norm_pass_pair_bytes": pair_bytes,
-        "traffic_over_algorithmic": (zero_bytes + pair_bytes + scale_bytes) / st.psi_bytes if st.psi_bytes else None,
+        "zero_bytes": zero_bytes,
+        "window_bytes": window_bytes,
+        "traffic_over_algorithmic": (zero_bytes + window_bytes) / st.psi_bytes if st.psi_bytes else None,
         "hbm_peak_GBs": hbm,
     }
 
