@@ -94,9 +94,9 @@ struct Header {
     unsigned long long refine_updates;  // point-updates of the FP32 refinement passes
     unsigned long long df_updates;      // point-updates of the double-float passes
     long long psi_total;                // psi doubles of the batch (level setup)
-    unsigned long long refine_max_updates;  // largest per-level point-updates of refine32
-    unsigned long long df_max_updates;      // largest per-level point-updates of newton_df / norm_df
-    int32_t refine_max_iters;               // most refine32 passes of one level
+    unsigned long long refine_max_updates;  // largest per-level FP32 point-updates
+    unsigned long long df_max_updates;      // largest per-level double-float point-updates
+    int32_t refine_max_iters;               // most FP32 passes of one level
     int32_t pad_hdr;
     int32_t hist[kLists * kBuckets];        // levels by list and window length
     unsigned long long long32_updates;      // CTA levels: FP32 pass point-updates

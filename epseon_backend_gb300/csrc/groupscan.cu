@@ -14,7 +14,7 @@
 //     64 x 16384 points, 8192              0.21 ms    0.59 ms
 //     48 x 4096..32768 points, 4096        0.14 ms    0.55 ms
 //     24 x 6000 points                     0.09 ms    0.16 ms
-//     1 x 10007 points, 1024 (all of them) 0.030 ms   0.133 ms
+//     1 x 10007 points, 1024 (all of them) 0.030 ms   0.133 ms  (static_scan.cu)
 // Larger batches keep the lane kernels, which their many energies fill (a warp
 // pass costs about twice a lane march's instructions per point), and so do
 // under-resolved potentials (fragile.cu), in full and beside these kernels: the

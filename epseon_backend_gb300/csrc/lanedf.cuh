@@ -265,7 +265,7 @@ __device__ __forceinline__ bool norm_df_level(const DevBatch& b, int slot) {
     const float2* Wf = b.Wf2 + m.offf;
     const double* W = b.W64 + m.off;
     // with psi requested every pass also stores its unnormalised psi-hat
-    // in the level's row; scale_psi applies the constants afterwards
+    // in the level's row; finish_row applies the constants afterwards
     double* row = psi_row(b, m, w);
     int n_pass = 0;
     auto pass = [&](int kk) {

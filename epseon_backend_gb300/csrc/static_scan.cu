@@ -36,6 +36,16 @@ namespace epscu {
 
 constexpr int kStaticMaxPoints = 65536;  // multiple of the scan's largest tile (4096)
 
+// A warp per trial energy (groupscan.cu) while that is faster than a lane per
+// energy, whose march of the whole grid takes the same time for any number of
+// energies that fits the chip.  The whole call, us, lanes / warps:
+//     points    1024 energies    4096        8192
+//      2500        75 / 56      75 / 98     74 / 124
+//     10007       180 / 74     180 / 157   179 / 224
+//     40000       587 / 120    589 / 340   588 / 471
+//     65536       933 / 151    934 / 451   936 / 634
+constexpr bool warp_counts(int64_t N, int64_t n_trial) { return n_trial * (7500 + N) <= 9500 * N; }
+
 struct StaticScanScratch {
     double W64[kStaticMaxPoints];
     unsigned long long Bkey[kStaticMaxPoints / 32];
@@ -151,8 +161,12 @@ extern "C" epscu_status epscu_count_levels_static(const double* V, int32_t N, do
     static_init_kernel<<<1, 1, 0, s>>>(S, r_min, r_max, mu, e_cap, N, n_trial);
     launch_prepare(b, s);
     const ScanShape shape{256, 2048, 3, 0};
-    launch_count_stride(b, 1, sm_count, s);
-    launch_scan_under(b, shape, sm_count, s);  // (an under-resolved grid's counts)
+    if (warp_counts(N, n_trial)) {
+        launch_count_stride(b, 1, sm_count, s);
+        launch_scan_under(b, shape, sm_count, s);  // (an under-resolved grid's counts)
+    } else {
+        launch_scan32(b, shape, sm_count, s);
+    }
     static_finish_kernel<<<1, 1024, 0, s>>>(S, n_trial, counts);
     e = cudaGetLastError();
     if (e != cudaSuccess) return static_fail(EPSCU_ERR_CUDA, cudaGetErrorString(e));

@@ -6,7 +6,10 @@ everything of an under-resolved potential equal to the last bit, since it takes
 the lane scan either way.  Trial ladders around the coarse stride (16), grids
 around one strip per lane (512 points) and on either side of the line where an
 energy takes a whole CTA (65536 points), and a batch on either side of the
-bisection scan's line (512)."""
+bisection scan's line (512).  The static count on either side of the line where
+it turns from a warp to a lane per energy: the levels below each trial energy,
+except within 1e-8 Hartree of a level, where FP32 counts may fall on either
+side."""
 from __future__ import annotations
 
 import numpy as np
@@ -67,3 +70,28 @@ def test_long_grids(ctx, N):
     b = synth.morse_batch(B=2, N=N, seed=9)
     levels, _ = _same(ctx, b.potentials(), b.r_min, b.r_max, b.mu, b.e_cap, 700)
     assert levels > 0
+
+
+@pytest.mark.parametrize("N, n_trial", [(2048, 1), (2500, 2375), (2500, 2376), (10007, 5430), (10007, 5431), (10007, 8192),
+                                        (65536, 300)])
+def test_static_counts_either_side_of_the_line(ctx, N, n_trial):
+    import ctypes as C
+
+    import torch
+
+    b = synth.morse_batch(B=1, N=N, seed=60)
+    V = np.ascontiguousarray(b.V(0))
+    args = (float(b.r_min[0]), float(b.r_max[0]), float(b.mu[0]), float(b.e_cap[0]))
+    sol = ctx.solve([V], *args, 2048, method=capi.METHOD_FAST_FP32C, level_capacity=300)
+    E = sol.energy[0, : int(sol.n_out[0])]
+    e_lo = V.min()
+    Ej = e_lo + (np.arange(n_trial) + 1) * ((args[3] - e_lo) / n_trial)
+    near = np.min(np.abs(Ej[:, None] - E[None, :]), axis=1) < 1e-8
+    Vd = torch.from_numpy(V).cuda()
+    counts = torch.full((n_trial,), -1, dtype=torch.int32, device="cuda")
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    rc = capi.load().epscu_count_levels_static(C.cast(C.c_void_p(Vd.data_ptr()), capi._dp), N, *args, n_trial,
+                                               C.cast(C.c_void_p(counts.data_ptr()), capi._ip), stream)
+    assert rc == 0
+    assert E.size > 0
+    assert np.array_equal(counts.cpu().numpy()[~near], np.searchsorted(E, Ej)[~near])
