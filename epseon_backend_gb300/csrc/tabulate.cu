@@ -4,8 +4,15 @@
 //
 // Everything is FP64, and on GB300 a FP64 instruction costs a warp 60 times an
 // FP32 one's issue: the kernels are bound by the FP64 pipes (one instruction
-// per point is 0.06 ms on the 2048-potential mixed batch, the write 0.05 ms),
-// so the work per point is cut to what the formulas need:
+// per point is 0.06 ms on the 2048-potential mixed batch, the write 0.05 ms).
+// The values are the plain formulas' on tiles of points (a solve on an
+// under-resolved grid amplifies their last bits, so no cheaper form of the
+// exponential or the divisions is used), with the spline's Thomas sweeps by
+// chunks: the LU recurrences contract by 2 - sqrt(3) = 0.268 a knot, so a lane
+// starts them before its chunk instead of waiting for the whole sweep (a serial
+// sweep by one thread, with a division a knot, was 1.2 ms of a launch whatever
+// its size).  The adjoint, whose sums have no such readers, cuts the work per
+// point:
 //   * the Morse exponential is geometric along a uniform grid: the product of a
 //     factor per 64-point block and a table of 64 factors (1 multiply instead of
 //     an exp a point);
@@ -13,13 +20,10 @@
 //   * the spline's interval and offset of point i by integer arithmetic
 //     (i (K - 1) = j (N - 1) + rem, u = rem / (N - 1)) and its cubic weights
 //     in factored form, w^3 - w = -u w (1 + w);
-//   * the spline's tridiagonal system (1, 4, 1) by chunks: the LU recurrences
-//     contract by 2 - sqrt(3) = 0.268 a knot, so a thread starts them
-//     kWarm = 40 knots before its chunk (0.268^40 = 1e-23) instead of waiting
-//     for the whole sweep (a serial sweep by one thread, with a division a
-//     knot, was 1.2 ms of a launch whatever its size).
-// Measured on the mixed batch (2048 potentials, 36.8 M points): tabulate 3.36 ->
-// 0.99 ms (knots 0.21), its adjoint 4.30 -> 1.44 ms.
+//   * the tridiagonal system (1, 4, 1) by chunks, kWarm = 40 knots before each
+//     (0.268^40 = 1e-23).
+// Measured on the mixed batch (2048 potentials, 36.8 M points): values and
+// adjoint together 7.8 -> 3.7 ms, the adjoint 4.30 -> 1.44 of them.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
@@ -33,6 +37,7 @@ namespace {
 
 constexpr int kTabThreads = 256;
 constexpr int kWarm = 40;
+constexpr int kSweepWarm = 160;
 constexpr int kBlock = 64;  // points per factor of the geometric exponential
 
 // 1/r: recip64 where its FP32 steps hold, the division elsewhere
@@ -98,7 +103,6 @@ __global__ void __launch_bounds__(kTabThreads) knots_kernel(const int32_t* kind,
     __shared__ double cp[kPivots + 1];
     const int p = blockIdx.x;
     if (kind[p] != EPSCU_KIND_SPLINE) return;
-    if (threadIdx.x <= kPivots) cp[threadIdx.x] = pivot_inverse(threadIdx.x);
     const double* P = params + (int64_t)p * 12;
     double* y = scratch + (int64_t)p * 4 * K;
     double* M = y + K;
@@ -107,12 +111,38 @@ __global__ void __launch_bounds__(kTabThreads) knots_kernel(const int32_t* kind,
     const double r0 = r_min[p], hk = (r_max[p] - r0) / (double)(K - 1);
     for (int j = threadIdx.x; j < K; j += kTabThreads) y[j] = knot_value(P, r0 + j * hk);
     __syncthreads();
-    // (the second derivative times hk^2 / 6 is what the evaluation uses)
+    // the Thomas sweeps by one warp, a chunk a lane: started kSweepWarm knots
+    // outside its chunk a sweep has the serial one's value to 1e-23 after 40 of
+    // them and, since two neighbouring numbers fall together with probability
+    // 0.73 a knot, its bits after the rest (but for a point in 10^4; the values a
+    // solve of an under-resolved grid gets should not depend on the chunks)
     const int n = K - 2;
-    for (int i = threadIdx.x; i < n; i += kTabThreads) rhs[i] = y[i + 2] - 2.0 * y[i + 1] + y[i];
-    if (threadIdx.x == 0) M[0] = M[K - 1] = 0.0;
+    const double s6 = 6.0 / (hk * hk);
+    if (threadIdx.x == 0) {
+        M[0] = M[K - 1] = 0.0;
+        cp[0] = 1.0 / 4.0;
+        for (int i = 1; i <= kPivots; ++i) cp[i] = 1.0 / (4.0 - cp[i - 1]);  // (its limit from 20 on)
+    }
+    for (int i = threadIdx.x; i < n; i += kTabThreads) rhs[i] = s6 * (y[i + 2] - 2.0 * y[i + 1] + y[i]);
     __syncthreads();
-    solve_141(rhs, d, M + 1, n, cp);
+    if (threadIdx.x >= 32) return;
+    const int per = (n + 31) / 32;
+    const int lo = min((int)threadIdx.x * per, n), hi = min(lo + per, n);
+    if (lo < hi) {
+        double v = 0.0;
+        for (int i = max(0, lo - kSweepWarm); i < hi; ++i) {
+            v = i == 0 ? rhs[0] / 4.0 : (rhs[i] - v) / (4.0 - cp[min(i - 1, kPivots)]);
+            if (i >= lo) d[i] = v;
+        }
+    }
+    __syncwarp();
+    if (lo < hi) {
+        double v = 0.0;
+        for (int i = min(n, hi + kSweepWarm) - 1; i >= lo; --i) {
+            v = i == n - 1 ? d[i] : d[i] - cp[min(i, kPivots)] * v;
+            if (i < hi) M[i + 1] = v;
+        }
+    }
 }
 
 // Interval and offset of grid point i on K knots: i (K - 1) = j (N - 1) + rem.
@@ -132,7 +162,6 @@ __global__ void __launch_bounds__(kTabThreads) tabulate_kernel(int32_t n, const 
                                                                const double* r_min, const double* r_max,
                                                                const int32_t* tiles, int32_t K, const double* scratch,
                                                                double* V) {
-    __shared__ double s_q[kBlock], s_b[kTabTile / kBlock];
     __shared__ int s_p;
     if (threadIdx.x == 0) {
         int lo = 0, hi = n - 1;  // the last p with tiles[p] <= blockIdx.x
@@ -155,47 +184,32 @@ __global__ void __launch_bounds__(kTabThreads) tabulate_kernel(int32_t n, const 
     if (k == EPSCU_KIND_SPLINE) {
         const double* y = scratch + (int64_t)p * 4 * K;
         const double* M = y + K;
-        const double inv = 1.0 / (double)(N - 1);
-        // kTabThreads points on: the interval advances by dj, the remainder by dr
-        const KnotPos step = {(int)((long long)kTabThreads * (K - 1) / (N - 1)),
-                              (int)((long long)kTabThreads * (K - 1) % (N - 1))};
-        KnotPos at = knot_pos(first + threadIdx.x, N, K);
+        const double hk = (r1 - r0) / (double)(K - 1);
+        const double h2 = hk * hk / 6.0;
         for (int x = threadIdx.x; x < count; x += kTabThreads) {
-            const double u = (double)at.rem * inv, w = 1.0 - u;
-            const double lin = fma(u, y[at.j + 1], w * y[at.j]);
-            const double cub = fma(1.0 + u, M[at.j + 1], (1.0 + w) * M[at.j]);
-            out[x] = fma(-(u * w), cub, lin);
-            at.j += step.j;
-            at.rem += step.rem;
-            if (at.rem >= N - 1) {
-                at.rem -= N - 1;
-                ++at.j;
-            }
-            if (at.j > K - 2) {  // the last point ends the last interval
-                at.rem += (at.j - (K - 2)) * (N - 1);
-                at.j = K - 2;
-            }
+            const int i = (int)first + x;
+            const double r = r0 + i * h;
+            const double t = (r - r0) / hk;
+            int j = (int)floor(t);
+            j = max(0, min(j, K - 2));
+            const double u = t - j, w = 1.0 - u;
+            out[x] = w * y[j] + u * y[j + 1] + h2 * ((w * w * w - w) * M[j] + (u * u * u - u) * M[j + 1]);
         }
     } else if (k == EPSCU_KIND_LJ) {
         const double eps = P[0], sigma = P[1];
         for (int x = threadIdx.x; x < count; x += kTabThreads) {
-            const double r = fma((double)(first + x), h, r0);
-            const double s = sigma * recip_r(r);
+            const int i = (int)first + x;
+            const double r = r0 + i * h;
+            const double s = sigma / r;
             const double s2 = s * s;
             const double s6 = s2 * s2 * s2;
-            out[x] = fma(4.0 * eps, fma(s6, s6, -s6), eps);
+            out[x] = 4.0 * eps * (s6 * s6 - s6) + eps;
         }
     } else {
-        const double De = P[0], a = P[1], re = P[2];
-        if (threadIdx.x < kBlock) s_q[threadIdx.x] = exp(-a * (threadIdx.x * h));
-        else if (threadIdx.x < kBlock + kTabTile / kBlock) {
-            const int b = threadIdx.x - kBlock;
-            s_b[b] = exp(-a * (fma((double)(first + b * kBlock), h, r0) - re));
-        }
-        __syncthreads();
         for (int x = threadIdx.x; x < count; x += kTabThreads) {
-            const double d = 1.0 - s_b[x / kBlock] * s_q[x % kBlock];
-            out[x] = De * d * d;
+            const int i = (int)first + x;
+            const double d = 1.0 - exp(-P[1] * (r0 + i * h - P[2]));
+            out[x] = P[0] * d * d;
         }
     }
 }
