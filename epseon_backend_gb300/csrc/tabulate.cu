@@ -17,9 +17,7 @@
 //     factor per 64-point block and a table of 64 factors (1 multiply instead of
 //     an exp a point);
 //   * 1/r by a FP32 reciprocal and two Newton steps;
-//   * the spline's interval and offset of point i by integer arithmetic
-//     (i (K - 1) = j (N - 1) + rem, u = rem / (N - 1)) and its cubic weights
-//     in factored form, w^3 - w = -u w (1 + w);
+//   * the spline's cubic weights in factored form, w^3 - w = -u w (1 + w);
 //   * the tridiagonal system (1, 4, 1) by chunks, kWarm = 40 knots before each
 //     (0.268^40 = 1e-23).
 // Measured on the mixed batch (2048 potentials, 36.8 M points): values and
@@ -143,17 +141,6 @@ __global__ void __launch_bounds__(kTabThreads) knots_kernel(const int32_t* kind,
             if (i < hi) M[i + 1] = v;
         }
     }
-}
-
-// Interval and offset of grid point i on K knots: i (K - 1) = j (N - 1) + rem.
-struct KnotPos {
-    int j, rem;
-};
-
-__device__ __forceinline__ KnotPos knot_pos(long long i, int N, int K) {
-    const long long t = i * (K - 1);
-    const int j = (int)min(t / (N - 1), (long long)K - 2);
-    return {j, (int)(t - (long long)j * (N - 1))};
 }
 
 // Values on the grid: one CTA per (potential, kTabTile points).
