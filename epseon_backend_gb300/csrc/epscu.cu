@@ -649,7 +649,10 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
                   (void*)o_e, (void*)o_nt, (void*)o_no, (void*)o_nd, (void*)o_st, (void*)o_err,
                   (long long)b.psi_capacity, method, cap, shape.threads, shape.tile, shape.stages, opts.tol,
                   (void*)s);  // s is the context's own stream
-    keybuf_extra = std::to_string(b.long_window) + "|" + std::to_string(b.wait_polls) + "|" + std::to_string(b.max_iter);
+    // (the grid lengths enter the captured launches by the set-up's tiles and by
+    // the longest grid: scan groups, cluster list, twist samples)
+    keybuf_extra = std::to_string(b.long_window) + "|" + std::to_string(b.wait_polls) + "|" + std::to_string(b.max_iter) +
+                   "|" + std::to_string(b.prep_tiles) + "|" + std::to_string(b.max_N);
     const std::string gkey = std::string(keybuf) + "|" + std::to_string(total_points) + "|" + keybuf_extra;
 
     auto enqueue_inputs = [&]() -> cudaError_t {
