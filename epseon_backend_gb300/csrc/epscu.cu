@@ -870,9 +870,8 @@ extern "C" epscu_status epscu_adjoint(epscu_ctx* ctx, const double* dL_dE, doubl
         b.psi_capacity = ctx->last_psi_total;
         // the writer of the solve's own method (its norm constants belong to it)
         if (ctx->last_method == EPSCU_METHOD_FAST_FP32C) {
-            EPSCU_CU(cudaMemsetAsync(&b.hdr->queue[kQWarpRewrite], 0, sizeof(int32_t), s));
-            EPSCU_CU(cudaMemsetAsync(&b.hdr->queue[kQLongRewrite], 0, sizeof(int32_t), s));
-            EPSCU_CU(cudaMemsetAsync(&b.hdr->queue[kQFragileRewrite], 0, sizeof(int32_t), s));
+            // (the last solve's queues have no other reader left)
+            EPSCU_CU(cudaMemsetAsync(b.hdr->queue, 0, sizeof(b.hdr->queue), s));
             launch_rewrite(b, ctx->sm_count, s);
             launch_fragile_rewrite(b, ctx->sm_count, s);
         } else {
