@@ -118,8 +118,8 @@ enum { kQBisect64 = 0, kQNorm64, kQWrite64, kQWarpLevels, kQLongLevels, kQRepair
 // (fragile.cu) the lane Newton handed the level over: its refinement, norm pass
 // and rewrite run on a CTA (the lane passes skip it)
 #define EPSCU_STATUS_FALLBACK 0x10000
-// (potential) a point inside the cut-offs lies above them: 1 + T can be small
-// there, and a fast pass renormalises after every point
+// (potential) a point inside the cut-offs lies above them: 1 + T can be small or
+// negative there, and a fast pass renormalises after every point
 #define EPSCU_STATUS_STEEP 0x40000
 #define EPSCU_STATUS_PUBLIC 0xffff
 // spacing of the samples of the twist-index search

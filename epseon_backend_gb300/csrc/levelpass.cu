@@ -82,10 +82,10 @@ __device__ __noinline__ PassDF norm_pass(const Grp<NW> G, const Chunk& c, const 
     PsiTag tag = psi_tag(s.e);
     SqSum ss;
     ss.init();
-    int nodes = 0, last = 0, flip = 0;
+    int nodes = 0, flip = 0, below = 0;
     int pk_L = -(1 << 30), pk_i = k;
     for_points(
-        c, Wf, [&](float2 w) { return df_point<true>(aE, w, c.steep); },
+        c, Wf, [&](float2 w, auto steep) { return df_point<true, steep.value>(aE, w); },
         [&](const PointDF& pt, float2* slot, int i) {
             const dfl psi = df_mul(s.u, pt.r);
             const float p = __fmul_rn(psi.h, psi.h);
@@ -96,9 +96,9 @@ __device__ __noinline__ PassDF norm_pass(const Grp<NW> G, const Chunk& c, const 
             df_march(pt.q, s.u, s.d);
             flip = (int)((__float_as_uint(s.u.h) ^ __float_as_uint(before)) >> 31);
             nodes += flip;
-            last = i;
         },
-        [&]() {
+        [&](const PointDF& pt, float2*, int i, auto steep) {
+            if (steep.value) below += pt.r.h < 0.0f;
             const float mm = fmaxf(fabsf(s.u.h), fabsf(s.d.h));
             if (mm > 0.0f && mm < INFINITY) {
                 const int e = exp_clamped(mm, 120);
@@ -113,7 +113,7 @@ __device__ __noinline__ PassDF norm_pass(const Grp<NW> G, const Chunk& c, const 
                 const int L = fexp(s.u.h) + s.e;
                 if (L > pk_L) {
                     pk_L = L;
-                    pk_i = last;
+                    pk_i = i;
                 }
             }
         },
@@ -140,7 +140,7 @@ __device__ __noinline__ PassDF norm_pass(const Grp<NW> G, const Chunk& c, const 
     // The start state's sign holds.
     if (c.ns > 0 && t != c.Lo - 1 && t != c.Lo + c.Li - 1 && neg != ((__float_as_uint(s.u.h) >> 31) != 0))
         nodes += flip ? -1 : 1;
-    nodes = __reduce_add_sync(full, nodes);
+    nodes = __reduce_add_sync(full, nodes - below);
     const DfE mine = c.ns > 0 ? sqsum_dfe(ss, 2 * s.e) : DfE{{0.0f, 0.0f}, 0};
     DfE so = warp_sum_dfe(out ? mine : DfE{{0.0f, 0.0f}, 0});
     DfE si = warp_sum_dfe(out ? DfE{{0.0f, 0.0f}, 0} : mine);
@@ -202,8 +202,8 @@ __device__ __noinline__ PassDF norm_pass(const Grp<NW> G, const Chunk& c, const 
     if (NW == 1 || G.warp() == 0) {
         double fk;
         r.gamma = gamma64(__dsub_rn(__dmul_rn(a, E), Wk), Eo, Ei, fk);
-        r.nodes = nodes;
-        r.count = nodes + (r.gamma < 0.0 ? 1 : 0);
+        r.nodes = nodes - (fk < 0.0 ? 1 : 0);
+        r.count = r.nodes + (r.gamma < 0.0 ? 1 : 0);
         const double rfk = 1.0 / fk;
         r.pk_out = df_to_double(Eo.u) * rfk;
         r.pk_in = df_to_double(Ei.u) * rfk;
@@ -280,7 +280,9 @@ struct States {
 
     __device__ __forceinline__ void run(const Grp<NW>& G, const Level& L, double E, int k, SharedDF<NW>& sh) {
         c = make_chunk(G.t(), Grp<NW>::kThreads, L.j0, L.j1, k, L.steep);
-        states_df<NW>(G, c, L.Wf, df_from_double(__dmul_rn(L.a, E)), sh, X, Eo, Ei, nodes, neg);
+        const double aE = __dmul_rn(L.a, E);
+        states_df<NW>(G, c, L.Wf, df_from_double(aE), sh, X, Eo, Ei, nodes, neg);
+        if (L.steep) nodes -= __dsub_rn(aE, __ldg(L.W + k)) < -1.0;  // (f < 0 at k)
     }
 
     // run() and the Cooley correction at its match point, with the sum of an
@@ -421,7 +423,7 @@ __device__ __forceinline__ int twist_point(const Grp<NW>& G, const Level& L, dou
         states_df<NW>(G, c, L.Wf, aE, sh, X, Eo, Ei, nodes, neg);
         dfl u = X.u, d = X.d;
         for_points(
-            c, L.Wf, [&](float2 w) { return df_point<false>(aE, w, c.steep); },
+            c, L.Wf, [&](float2 w, auto steep) { return df_point<false, steep.value>(aE, w); },
             [&](const PointDF& pt, float2*, int i) {
                 const int rel = i - L.j0;
                 if (rel % kTwistSample == 0 && rel / kTwistSample < stride) {
@@ -443,7 +445,7 @@ __device__ __forceinline__ int twist_point(const Grp<NW>& G, const Level& L, dou
                 }
                 df_march(pt.q, u, d);
             },
-            [&]() {
+            [&](const PointDF&, float2*, int, auto) {
                 const int e = exp_clamped(fmaxf(fabsf(u.h), fabsf(d.h)), 120);
                 const float sc = fpow2(-e);
                 u = df_scale(u, sc);
