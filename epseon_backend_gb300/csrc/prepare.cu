@@ -159,7 +159,7 @@ __device__ __forceinline__ int halvings_to(double delta, double tol) {
 __device__ void finish_potential(const DevBatch& b, int p, int nt, const PrepTile* rec) {
     __shared__ unsigned long long s_k[3][kPrepThreads / 32];
     __shared__ int s_i[4][kPrepThreads / 32];
-    __shared__ unsigned long long s_kt;
+    __shared__ unsigned long long s_kt, s_kb;
     __shared__ double s_delta, s_kmax;
     __shared__ int s_K;
     constexpr int nw = kPrepThreads / 32;
@@ -206,6 +206,7 @@ __device__ void finish_potential(const DevBatch& b, int p, int nt, const PrepTil
     if (tid == 32) {  // (beside it)
         s_delta = __ddiv_rn(__dsub_rn(m.e_cap, vmin), (double)m.n_trial);
         s_kmax = sqrt(2.0 * m.mu * (m.e_cap - vmin));
+        s_kb = dkey0(__dadd_rn(vmin, __ddiv_rn(1.0 - 1e-6, m.a)));
         s_K = halvings_to(s_delta, b.tol > 0.0 ? b.tol : 1e-12);
     }
     __syncthreads();
@@ -251,23 +252,26 @@ __device__ void finish_potential(const DevBatch& b, int p, int nt, const PrepTil
     const int i0 = first < 1 ? 1 : first;
     const int i1 = last > N - 2 ? N - 2 : last;
 
-    // a barrier inside the cut-offs that rises above them, and the minima of
-    // the two end tiles over [i0, i1]
+    // a barrier inside the cut-offs that rises above them (1), or to where f is
+    // negative (2; from 1e-6 below, for the rounding of T), and the minima of the
+    // two end tiles over [i0, i1]
+    const unsigned long long kb = s_kb;
+    auto above = [&](unsigned long long k) { return (k > kt ? 1 : 0) | (k > kb ? 2 : 0); };
     int steep = 0;
     unsigned long long ka = kKeyMax, kz = kKeyMax;
-    for (int t = ft + 1 + tid; t < lt; t += kPrepThreads) steep |= rec[t].kmax > kt;
+    for (int t = ft + 1 + tid; t < lt; t += kPrepThreads) steep |= above(rec[t].kmax);
     if (lt >= 0)
         for (int x = tid; x < kPrepTile; x += kPrepThreads) {
             const int i = ft * kPrepTile + x, j = lt * kPrepTile + x;
             if (i >= i0 && i <= i1) {
                 const unsigned long long k = dkey0(V[i]);
                 ka = min(ka, k);
-                steep |= k > kt;
+                steep |= above(k);
             }
             if (j >= i0 && j <= i1) {
                 const unsigned long long k = dkey0(V[j]);
                 kz = min(kz, k);
-                steep |= k > kt;
+                steep |= above(k);
             }
         }
     ka = warp_min_key(ka);
@@ -302,6 +306,7 @@ __device__ void finish_potential(const DevBatch& b, int p, int nt, const PrepTil
     m.n_bisect = s_K;
     if (s_kmax * m.h > 1.0) status |= EPSCU_STATUS_UNDER;
     if (steep) status |= EPSCU_STATUS_STEEP;
+    if (steep & 2) status |= EPSCU_STATUS_BELOW;
     m.status = status;
     if (b.under_list && (status & EPSCU_STATUS_UNDER) && !(status & EPSCU_STATUS_BAD))
         b.under_list[atomicAdd(&b.hdr->n_under, 1)] = p;

@@ -173,6 +173,26 @@ __device__ __forceinline__ void step32(float l, float c, float& A, float& D, int
     A = An;
 }
 
+// One step of a potential with points where f < 0 (EPSCU_STATUS_BELOW): a sign
+// change of A there is none of u, and the point itself is no level
+// (grouppass.cuh), so it counts -1 instead of 1.  Renormalised after every
+// point, where A grows up to 12 |T|-fold.
+__device__ __forceinline__ void step32_below(float T, float& A, float& D, int& nodes) {
+    const float X = fmaf(-12.0f, A, D);
+    D = fmaf(T, X, D);
+    const float An = A + fmaf(T, A, D);
+    const int flip = (int)((__float_as_uint(An) ^ __float_as_uint(A)) >> 31);
+    nodes += T < -1.0f ? -flip : flip;
+    A = An;
+    renorm_f(A, D);
+}
+
+// whether a potential's counts take it (an under-resolved one's levels keep the
+// lane passes' counts, fragile.cu)
+__device__ __forceinline__ bool counts_below(const PotMeta& m) {
+    return (m.status & (EPSCU_STATUS_BELOW | EPSCU_STATUS_UNDER)) == EPSCU_STATUS_BELOW;
+}
+
 // Step with the sign of A shifted into a bit history (one funnel shift per
 // step; the sign changes are popcounted once per 16-step chunk).
 __device__ __forceinline__ void step32b(float l, float c, float& A, float& D, uint32_t& bits) {
@@ -222,8 +242,13 @@ __device__ __forceinline__ void chunk16_down(const float* __restrict__ c, float 
 
 // points a0..a1 (a0 <= a1) of tile tb (first point T0), ascending
 __device__ __forceinline__ void run_up(const float* __restrict__ tb, int T0, int a0, int a1, float l, float& A,
-                                       float& D, int& nodes) {
+                                       float& D, int& nodes, bool below) {
     int i = a0;
+    if (below) {
+#pragma unroll 1
+        for (; i <= a1; ++i) step32_below(tb[i - T0] + l, A, D, nodes);
+        return;
+    }
     for (; i <= a1 && (i & 15); ++i) step32(l, tb[i - T0], A, D, nodes);
     renorm_f(A, D);
     uint32_t bits = __float_as_uint(A) >> 31;
@@ -233,8 +258,13 @@ __device__ __forceinline__ void run_up(const float* __restrict__ tb, int T0, int
 
 // points a0..a1 (a0 >= a1) of tile tb, descending
 __device__ __forceinline__ void run_down(const float* __restrict__ tb, int T0, int a0, int a1, float l, float& A,
-                                         float& D, int& nodes) {
+                                         float& D, int& nodes, bool below) {
     int i = a0;
+    if (below) {
+#pragma unroll 1
+        for (; i >= a1; --i) step32_below(tb[i - T0] + l, A, D, nodes);
+        return;
+    }
     for (; i >= a1 && ((i & 15) != 15); --i) step32(l, tb[i - T0], A, D, nodes);
     renorm_f(A, D);
     uint32_t bits = __float_as_uint(A) >> 31;
@@ -346,6 +376,7 @@ __global__ void __launch_bounds__(THREADS) scan32_kernel(DevBatch b, int ipp, in
         const float H = __double2float_rn(__dmul_rn(m.a, trial_energy(m, sel(blk * THREADS + THREADS / 2))));
         const float l = __double2float_rn(aE - (double)H);
         const int k = m.k_scan;
+        const bool below = counts_below(m);
         float A = 1.0f, D = 1.0f;  // u_{j0} = 1, u_{j0-1} = 0
         float Ao = 1.0f, Do = 1.0f;
         int nodes = 0;
@@ -382,7 +413,7 @@ __global__ void __launch_bounds__(THREADS) scan32_kernel(DevBatch b, int ipp, in
             const int T0 = seq.tile(t) * TILE;
             if (t < seq.n_out) {
                 const int a0 = max(j0, T0), a1 = min(k - 1, T0 + TILE - 1);
-                run_up(conv, T0, a0, a1, l, A, D, nodes);
+                run_up(conv, T0, a0, a1, l, A, D, nodes, below);
             } else {
                 if (!inward) {
                     inward = true;
@@ -392,7 +423,7 @@ __global__ void __launch_bounds__(THREADS) scan32_kernel(DevBatch b, int ipp, in
                     D = 1.0f;
                 }
                 const int a0 = min(j1, T0 + TILE - 1), a1 = max(k + 1, T0);
-                run_down(conv, T0, a0, a1, l, A, D, nodes);
+                run_down(conv, T0, a0, a1, l, A, D, nodes, below);
             }
             __syncthreads();  // every thread is done with conv
         }
@@ -560,8 +591,13 @@ __device__ __forceinline__ void step32tb(float aEh, float aEl, float wx, float w
 
 // points a0..a1 ascending (a0 <= a1) of a raw tile tb whose first point is T0
 __device__ __forceinline__ void run_up_raw(const float2* __restrict__ tb, int T0, int a0, int a1, float aEh, float aEl,
-                                           float& A, float& D, int& nodes) {
+                                           float& A, float& D, int& nodes, bool below) {
     int i = a0;
+    if (below) {
+#pragma unroll 1
+        for (; i <= a1; ++i) step32_below((aEh - tb[i - T0].x) + (aEl - tb[i - T0].y), A, D, nodes);
+        return;
+    }
     for (; i <= a1 && (i & 15); ++i) step32t(aEh, aEl, tb[i - T0], A, D, nodes);
     renorm_f(A, D);
     uint32_t bits = __float_as_uint(A) >> 31;
@@ -581,8 +617,13 @@ __device__ __forceinline__ void run_up_raw(const float2* __restrict__ tb, int T0
 
 // points a0..a1 descending (a0 >= a1)
 __device__ __forceinline__ void run_down_raw(const float2* __restrict__ tb, int T0, int a0, int a1, float aEh,
-                                             float aEl, float& A, float& D, int& nodes) {
+                                             float aEl, float& A, float& D, int& nodes, bool below) {
     int i = a0;
+    if (below) {
+#pragma unroll 1
+        for (; i >= a1; --i) step32_below((aEh - tb[i - T0].x) + (aEl - tb[i - T0].y), A, D, nodes);
+        return;
+    }
     for (; i >= a1 && ((i & 15) != 15); --i) step32t(aEh, aEl, tb[i - T0], A, D, nodes);
     renorm_f(A, D);
     uint32_t bits = __float_as_uint(A) >> 31;
@@ -653,6 +694,7 @@ __global__ void __launch_bounds__(kCountThreads) count_list_kernel(DevBatch b) {
         // outward: u_{j0} = 1, u_{j0-1} = 0; inward: v_{j1} = 1, v_{j1+1} = 0
         float A = 1.0f, D = 1.0f;
         int nodes = 0;
+        const bool below = counts_below(m);
         const TileSeq seq = make_seq(j0, j1, k, kCountTile);
         const int L = max(seq.n_out, seq.n_in);
         for (int t = 0; t < L; ++t) {
@@ -666,9 +708,11 @@ __global__ void __launch_bounds__(kCountThreads) count_list_kernel(DevBatch b) {
             __syncthreads();
             if (side == 0) {
                 if (To >= 0)
-                    run_up_raw(tile_o, To, max(j0, To), min(k - 1, To + kCountTile - 1), aEh, aEl, A, D, nodes);
+                    run_up_raw(tile_o, To, max(j0, To), min(k - 1, To + kCountTile - 1), aEh, aEl, A, D, nodes,
+                               below);
             } else if (Ti >= 0) {
-                run_down_raw(tile_i, Ti, min(j1, Ti + kCountTile - 1), max(k + 1, Ti), aEh, aEl, A, D, nodes);
+                run_down_raw(tile_i, Ti, min(j1, Ti + kCountTile - 1), max(k + 1, Ti), aEh, aEl, A, D, nodes,
+                             below);
             }
         }
         if (side == 1) {
