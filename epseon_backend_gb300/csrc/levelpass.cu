@@ -314,10 +314,12 @@ struct States {
 
 // The norm pass at E and its match-point candidates: the FP32 one, the peak
 // of |psi| seen by the pass, the outer turning point and its peak; the first
-// whose stitched solution has v nodes wins.  One more pass at E + dE when the
-// correction is above the energy's resolution (psi is only as accurate as its
-// energy).  `have`: st holds phase 1 at (E, k).  Writes the constants and the
-// energy into w.
+// whose stitched solution has v nodes wins.  (The peak itself, not the strip
+// boundary before it: that can lie behind a wall, where psi is 2^-17 of the peak
+// and the stitched solution off by the energy's rounding times that squared.)
+// One more pass at E + dE when the correction is above the energy's resolution
+// (psi is only as accurate as its energy).  `have`: st holds phase 1 at (E, k).
+// Writes the constants and the energy into w.
 template <int NW>
 __device__ __forceinline__ void norm_level(const Grp<NW>& G, const DevBatch& b, const Level& L, LevelWork& w, double E,
                                            int k, States<NW>& st, bool have, double* row, SharedDF<NW>& sh, int& n_pass,
@@ -341,7 +343,7 @@ __device__ __forceinline__ void norm_level(const Grp<NW>& G, const DevBatch& b, 
             best = r;
             k = kk;
             if (r.peak_log2 >= 2) {
-                kk = align_k(L.j0, L.j1, r.peak_i);
+                kk = clamp_k(w, r.peak_i);
                 if (kk != k) continue;  // step 1: the peak's point
             }
             step = 1;
@@ -350,7 +352,7 @@ __device__ __forceinline__ void norm_level(const Grp<NW>& G, const DevBatch& b, 
             k = kk;
         } else if (step == 2) {
             if (r.nodes != L.v && r.peak_log2 >= 1) {
-                kk = align_k(L.j0, L.j1, r.peak_i);
+                kk = clamp_k(w, r.peak_i);
                 continue;  // step 3: its peak
             }
             step = 3;
