@@ -790,9 +790,10 @@ __global__ void __launch_bounds__(128) window_kernel(DevBatch b) {
             k = match_index(m, b, w.E) & ~15;
             len = jw.y - jw.x;
             const int s = slot - m.level_base;
-            const bool fragile = (m.status & EPSCU_STATUS_UNDER) ||
-                                 w.n_in_bracket > 1 || (s > 0 && w.hi0 - b.levels[slot - 1].lo0 < kFragileGap) ||
-                                 (s + 1 < m.n_out && b.levels[slot + 1].hi0 - w.lo0 < kFragileGap);
+            const bool close = w.n_in_bracket > 1 || (s > 0 && w.hi0 - b.levels[slot - 1].lo0 < kFragileGap) ||
+                               (s + 1 < m.n_out && b.levels[slot + 1].hi0 - w.lo0 < kFragileGap);
+            // (where f can be negative the lane passes' counts are not the levels')
+            const bool fragile = (m.status & EPSCU_STATUS_UNDER) || (close && !(m.status & EPSCU_STATUS_BELOW));
             list = fragile ? (len > fragile_min ? kListFragileLong : kListFragile)
                            : (len > cluster_min ? kListCluster : len > long_min ? kListLong : kListWarp);
         }
