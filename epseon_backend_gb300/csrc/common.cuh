@@ -254,24 +254,27 @@ __device__ __forceinline__ int count64(const PotMeta& m, const double* __restric
     return nodes + count_join64(aE, __ldg(W + k), A, B, C, D);
 }
 
-// 1/f, of either sign (f = 1 + T is negative on a barrier with a (V - E) > 1):
-// FP32 reciprocal refined by two FP64 Newton steps (relative error at the FP64
-// rounding level).  Within 2^+-100 the two conversions run on the integer pipes
-// (exact, and the same rounding): magnitude there and back, the sign carried
-// beside it.
-__device__ __forceinline__ double recip64(double f) {
+// 1/f for 2^-100 <= |f| <= 2^100, of either sign: FP32 reciprocal refined by two
+// FP64 Newton steps (relative error at the FP64 rounding level).  The two
+// conversions run on the integer pipes (exact, and the same rounding): the
+// magnitude there and back, the sign put into the double (the bits above the
+// float's exponent fall off the first shift).
+__device__ __forceinline__ double recip64_normal(double f) {
     const unsigned long long u = (unsigned long long)__double_as_longlong(f);
-    const uint32_t top = (uint32_t)(u >> 32), sign = top & 0x80000000u;
-    double r;
-    if (((top >> 20) & 0x7ffu) - 923u > 200u) {
-        r = (double)__frcp_rn((float)f);
-    } else {
-        const uint32_t dropped = (uint32_t)u & 0x1fffffffu;
-        uint32_t b = (uint32_t)((u >> 29) - (896ull << 23)) & 0x7fffffffu;  // truncated to a float's bits
-        b += dropped > 0x10000000u || (dropped == 0x10000000u && (b & 1u));
-        const uint32_t x = __float_as_uint(__frcp_rn(__uint_as_float(b)));
-        r = __hiloint2double((int)(((x >> 3) + (896u << 20)) | sign), (int)(x << 29));
-    }
+    const uint32_t dropped = (uint32_t)u & 0x1fffffffu;
+    uint32_t b = (uint32_t)((u >> 29) - (896ull << 23));  // truncated to a float's bits
+    b += dropped > 0x10000000u || (dropped == 0x10000000u && (b & 1u));
+    const uint32_t x = __float_as_uint(__frcp_rn(__uint_as_float(b)));
+    double r = __hiloint2double((int)(((x >> 3) + (896u << 20)) | ((uint32_t)(u >> 32) & 0x80000000u)), (int)(x << 29));
+    r = __fma_rn(r, __fma_rn(-f, r, 1.0), r);
+    r = __fma_rn(r, __fma_rn(-f, r, 1.0), r);
+    return r;
+}
+
+// ... for any f: the conversions themselves outside that range
+__device__ __forceinline__ double recip64(double f) {
+    if ((((uint32_t)__double2hiint(f) >> 20) & 0x7ffu) - 923u <= 200u) return recip64_normal(f);
+    double r = (double)__frcp_rn((float)f);
     r = __fma_rn(r, __fma_rn(-f, r, 1.0), r);
     r = __fma_rn(r, __fma_rn(-f, r, 1.0), r);
     return r;

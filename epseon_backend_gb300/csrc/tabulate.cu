@@ -38,9 +38,9 @@ constexpr int kWarm = 40;
 constexpr int kSweepWarm = 160;
 constexpr int kBlock = 64;  // points per factor of the geometric exponential
 
-// 1/r: recip64 where its FP32 steps hold, the division elsewhere
+// 1/r: an FP32 reciprocal and Newton steps where they hold, the division elsewhere
 __device__ __forceinline__ double recip_r(double r) {
-    return fabs(r) > 1e-30 && fabs(r) < 1e30 ? recip64(r) : 1.0 / r;
+    return fabs(r) > 1e-30 && fabs(r) < 1e30 ? recip64_normal(r) : 1.0 / r;
 }
 
 // Knot value: Morse and up to three Gaussian bumps.

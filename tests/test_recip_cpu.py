@@ -1,7 +1,6 @@
-"""recip64 (csrc/common.cuh) restated on the CPU: the integer conversions to and
+"""recip64_normal (csrc/common.cuh) restated on the CPU: the integer conversions to and
 from the FP32 reciprocal give what the conversions themselves give, for either
-sign, at rounding ties and at significands that carry into the exponent; outside
-2^+-100 the conversions are used."""
+sign, at rounding ties and at significands that carry into the exponent."""
 from __future__ import annotations
 
 import numpy as np
@@ -13,7 +12,8 @@ def seed_by_bits(f: float) -> float:
     sign = top & 0x80000000
     assert not ((((top >> 20) & 0x7FF) - 923) & 0xFFFFFFFF) > 200
     dropped = u & 0x1FFFFFFF
-    b = ((u >> 29) - (896 << 23)) & 0x7FFFFFFF
+    b = ((u >> 29) - (896 << 23)) & 0xFFFFFFFF
+    assert b < 1 << 31
     b += 1 if dropped > 0x10000000 or (dropped == 0x10000000 and b & 1) else 0
     with np.errstate(all="ignore"):
         x = int((np.float32(1.0) / np.uint32(b).view(np.float32)).view(np.uint32))
