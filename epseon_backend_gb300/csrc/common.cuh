@@ -144,10 +144,11 @@ __device__ __forceinline__ void step64(double aE, double w, double& A, double& B
     A = An;
 }
 
-// x < 0 for a number, on the integer pipes: a FP64 comparison costs what a FP64
-// multiply-add does (64 cycles of its SM quarter's pipe a warp on GB300)
+// x < 0 on the integer pipes: a FP64 comparison costs what a FP64 multiply-add
+// does (64 cycles of its SM quarter's pipe a warp on GB300).  Above -0, up to
+// -inf: a NaN, which an overflowing march leaves with its sign bit set, is not.
 __device__ __forceinline__ bool negative(double x) {
-    return (unsigned long long)__double_as_longlong(x) > 0x8000000000000000ull;
+    return (unsigned long long)__double_as_longlong(x) - 0x8000000000000001ull < 0x7ff0000000000000ull;
 }
 
 // frexp-style exponent of |m| (m = f 2^e, f in [0.5, 1)) for finite normal m.
