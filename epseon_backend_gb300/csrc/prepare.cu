@@ -203,12 +203,12 @@ __device__ void finish_potential(const DevBatch& b, int p, int nt, const PrepTil
     }
     const double vmin = dkey_inv(kall);
     if (tid == 0) s_kt = cutoff_key(m.a, vmin, kall);
-    if (tid == 32) {  // (beside it)
+    if (tid == 32) {  // (beside it, as is the next)
         s_delta = __ddiv_rn(__dsub_rn(m.e_cap, vmin), (double)m.n_trial);
         s_kmax = sqrt(2.0 * m.mu * (m.e_cap - vmin));
-        s_kb = dkey0(__dadd_rn(vmin, __ddiv_rn(1.0 - 1e-6, m.a)));
         s_K = halvings_to(s_delta, b.tol > 0.0 ? b.tol : 1e-12);
     }
+    if (tid == 64) s_kb = dkey0(__dadd_rn(vmin, __ddiv_rn(1.0 - 1e-6, m.a)));
     __syncthreads();
     const unsigned long long kt = s_kt;
 
