@@ -51,6 +51,16 @@ constexpr int kCtaCtasPerSm = 2;
 // (Hartree); the energy after such a step is far inside their first step's
 // range
 constexpr double kTol32 = 3e-8;
+// a double-float correction at most this large (Hartree, relative above 1) is
+// left to the reported energy: psi keeps the energy it was computed at, and is
+// off by what is left over the gap to the next level.  psi's error in L2 against
+// FP64 at a bracket of 1e-15 (41137 levels of 1500 uneven grids; rms, median,
+// 99th percentile), and the solve of 2048 uneven grids with psi and gradient:
+//     1e-14     6.1e-12  3.2e-13  2.8e-11    17.4 ms
+//      2e-15    1.7e-12  2.2e-13  6.3e-12    17.8 ms
+//      1e-15    1.3e-12  1.9e-13  3.8e-12    17.9 ms
+// (the passes of a lane per level before these: 2.7e-12, 2.2e-13, 6.8e-12)
+constexpr double kSettled = 1e-15;
 // halvings before the repair kernel looks for a better match point (256 bumped
 // Morse wells: the kernel 1.0 ms without, 0.51 ms after 4, 0.39 ms after 2)
 constexpr int kHalveFirst = 2;
@@ -610,7 +620,7 @@ __device__ __forceinline__ void level_queue(const DevBatch& b, SharedDF<NW>& sh,
                 // (a correction at the energy's resolution: phase 3 goes on from
                 // this pass's states, and its own correction is added to E)
                 const double res = fmax(1.0, fabs(E));
-                if (fabs(dE) <= 1e-14 * res || (it >= 4 && fabs(dE) <= 1e-12 * res)) {
+                if (fabs(dE) <= kSettled * res || (it >= 4 && fabs(dE) <= 1e-12 * res)) {
                     settled = true;
                     break;
                 }
