@@ -795,11 +795,11 @@ extern "C" epscu_status epscu_solve(epscu_ctx* ctx, const epscu_batch* batch, ep
     st.norm_redos = hh->n_redo;
     const bool psi_on = want_psi || keep_psi || (alloc_psi && b.psi);
     st.psi_bytes = psi_on ? psi_total * 8 : 0;
-    // plain: prepare, scan64, level/unit setup, bracket, bisect64, norm64,
-    // twist64, gather (+ write64); fast: prepare, scan window, scan32, level
-    // setup, bracket, window, order, the two level kernels, repair, the two
-    // fragile kernels, gather
-    st.kernel_launches = method == EPSCU_METHOD_FAST_FP32C ? 13 : 9 + (psi_on ? 1 : 0);
+    // plain: prepare, block minima, scan64, level and unit setup, bracket,
+    // bisect64, norm64, twist64, gather (+ write64); fast: prepare, block minima,
+    // scan window, scan32, level setup, bracket, window, order, the level kernel
+    // (with clusters or without), repair, the two fragile kernels, gather
+    st.kernel_launches = method == EPSCU_METHOD_FAST_FP32C ? 13 : 10 + (psi_on ? 1 : 0);
     if (b.under_list) {  // the group scan's plan, count round and lane scan
         st.kernel_launches += 3;
     } else if (b.bis_list) {  // the plan + count rounds after the coarse scan32
