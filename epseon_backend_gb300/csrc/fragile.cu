@@ -1268,7 +1268,8 @@ __global__ void __launch_bounds__(256) fragile_zero_kernel(DevBatch b) {
     const int total = b.hdr->total_levels;
     for (int slot = warp; slot < total; slot += n_warps) {
         const LevelWork w = b.levels[slot];
-        if (w.bucket < kListFragile * kBuckets) continue;
+        const int list = w.bucket / kBuckets;
+        if (list != kListFragile && list != kListFragileLong) continue;
         const int N = b.meta[w.p].N;
         double* row = psi_row(b, b.meta[w.p], w);
         const bool none = no_result(w);
