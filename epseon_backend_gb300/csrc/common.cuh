@@ -191,7 +191,11 @@ constexpr int kBisectSplit = 16;
 constexpr int kBisectSingle = 4;
 // batches of at least this many potentials scan with a lane per energy (scan.cu;
 // smaller ones have too few energies to cover a lane's march of its window),
-// smaller ones with a group per energy (groupscan.cu)
+// smaller ones with a group per energy (groupscan.cu).  The solve of uneven grids
+// of 2048 to 65536 points, 8192 energies, ms, lanes / groups: 256 potentials 4.5 /
+// 3.2, 384 4.8 / 3.8, 512 5.2 / 4.5, 700 7.5 / 7.0, 1024 7.7 / 7.9, 2048 16.3 /
+// 17.8; of 2048 to 8192 points, 1024 energies: 256 2.8 / 3.0, 512 5.15 / 5.09,
+// 1024 11.2 / 11.2, 2048 13.5 / 14.1
 constexpr int kBisectMinPotentials = 512;
 
 // e-folds of decay at the ends of the fast method's windows: e^-36 = 2.3e-16,

@@ -37,7 +37,13 @@ __host__ __device__ __forceinline__ int default_long_window(int total_levels) {
 // of level passes; 37 levels on 65536 points, the solve 674 -> 487 us; 333
 // levels on 65536 points with the threshold at 16384 instead of 32768: 888
 // instead of 693 us, so it too rises with the number of levels).  Batches of
-// more than kClusterPotentials potentials have levels enough for the CTAs.
+// more than kClusterPotentials potentials take CTAs, which are as fast or faster
+// there unless each has very few levels.  The solve, us, clusters / CTAs, on
+// Morse grids of 65536 points:
+//     17 potentials,  958 levels   936 /  897      194 levels  1132 / 1024
+//     24             1056          977 /  937      211         1214 / 1259
+//     32             1591         1285 / 1210      318          951 / 1215
+//     48             2516         1708 / 1639      515         1410 / 1392
 constexpr int kMinClusterWindow = 16384;
 constexpr int kClusterLevels = 256;
 constexpr int kClusterPotentials = 16;
@@ -49,8 +55,15 @@ __host__ __device__ __forceinline__ int default_cluster_window(int total_levels)
 }
 
 // The threshold of the fragile levels' CTA passes (fragile.cu), which cost ~3x
-// the point-updates of a lane's but cut its latency ~80x: 8192 points at
-// >= ~9e4 levels, proportionally less below, never under 1024.
+// the point-updates of a lane's but cut its latency ~80x: 8192 points above 3e4
+// levels, proportionally less below, never under 1024.  The solve, us, by
+// threshold (uneven grids; the rule's choice in brackets):
+//     levels               1024    2048    4096    8192    16384
+//       705 (16 grids)    [569]             560              559
+//      2829 (48)          [999]            1325             1304
+//     11630 (256)         2666   [2732]    3153             6815
+//     25362 (512)         6170            [7135]           10150
+//     93060 (2048)       13016            12919  [14250]   15240
 constexpr int kFragileLongWindow = 8192;
 constexpr int kFragileLongLevels = 60000;
 constexpr int kFragileMinLongWindow = 1024;

@@ -7,16 +7,17 @@
 // device-resident solve (replayed when the same buffers are solved again).
 //
 // Solve pipeline:
-//   prepare -> scan (FP64 | FP32 TMA persistent; for batches of >= 512
-//   potentials the FP32 scan on every 16th trial energy, then a count round
-//   inside the cells where the counts change) -> level set-up + brackets
+//   prepare -> scan -> level set-up + brackets.  The plain method counts every
+//   trial energy in FP64; the fast one every 16th, then a count round inside the
+//   cells where the counts change: a lane per energy (FP32, TMA-staged) in
+//   batches of >= 512 potentials, a warp or CTA per energy in smaller ones.
 //   plain : bisect64 -> norm64 -> twist64 -> write64            (native FP64)
 //   fast  : window, order, then two branches on two streams (graph
-//           fork/join): levels<8> (a CTA per long level) and levels<1> (a
-//           warp per level), each taking a level through its FP32 passes, its
-//           double-float passes (FP64 matching and norm integral) and its psi
-//           row, then repair; beside them the fragile levels (fragile,
-//           fragile_repair)
+//           fork/join): levels (a cluster of CTAs, a CTA or a warp per level by
+//           window length; with clusters a kernel of its own), which takes a
+//           level through its FP32 passes, its double-float passes (FP64
+//           matching and norm integral) and its psi row, then repair; beside
+//           them the fragile levels (fragile, fragile_repair)
 //   -> gather into the caller's layout.
 #include <cuda_runtime.h>
 

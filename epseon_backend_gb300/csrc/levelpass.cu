@@ -694,13 +694,13 @@ __global__ void __cluster_dims__(kClusterWarps / kCtaWarps, 1, 1)
     level_queue<1>(b, sh1, sh321);
 }
 
-// Levels the queues above left over: first those stage 2 could not settle
-// (the FP32 bracket may be off by its count errors: safeguarded Cooley-Newton
-// with double-float passes from the FP32 stage's bracket, or the scan's widened
-// by one trial spacing where its ends do not hold; Newton steps only while the pass sees the level's own node count
-// and they stay inside the bracket, bisection otherwise), then those whose
-// final pass disagrees.  Their psi is a CTA group's from here on: they join
-// the long list, which rewrite<8> walks.
+// Levels the queues above left over: first those stage 2 could not settle (the
+// FP32 bracket may be off by its count errors: safeguarded Cooley-Newton with
+// double-float passes from the FP32 stage's bracket, or the scan's widened by
+// one trial spacing where its ends do not hold; Newton steps only while the pass
+// sees the level's own node count and they stay inside the bracket, bisection
+// otherwise), then those whose final pass disagrees.  Their psi is a CTA's from
+// here on: they join the long list, which the rewrite's CTAs walk.
 __global__ void __launch_bounds__(32 * kCtaWarps, kCtaCtasPerSm) repair_kernel(DevBatch b) {
     constexpr int NW = kCtaWarps;
     __shared__ SharedDF<NW> sh;
