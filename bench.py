@@ -40,12 +40,12 @@ UNIT = "levels/s"
 E_TOL = 1e-9
 CPU_SAMPLE = 96  # potentials of the workload the CPU legs time
 # dram__bytes_read.sum + dram__bytes_write.sum of one scan32 launch per grid
-# point, ncu on the 128-potential mixed batch (18.12 MB / 2,242,300 points)
-SCAN32_DRAM_BYTES_PER_POINT = 8.08
+# point, ncu on the 512-potential mixed batch (76.56 MB read / 8,861,352 points)
+SCAN32_DRAM_BYTES_PER_POINT = 8.64
 # ncu (dram__bytes_read.sum + dram__bytes_write.sum) of levels_kernel per
-# point-update on the 512-potential mixed batch (5.18 GB, the psi rows and the
-# windows' W, over 452,052,088 point-updates)
-LEVELS_DRAM_BYTES_PER_UPDATE = 11.5
+# point-update on the 512-potential mixed batch (5.23 GB, the psi rows and the
+# windows' W, over 481,633,175 point-updates)
+LEVELS_DRAM_BYTES_PER_UPDATE = 10.9
 
 
 def dist_env():
