@@ -121,11 +121,12 @@ enum { kQBisect64 = 0, kQNorm64, kQWrite64, kQWarpLevels, kQLongLevels, kQRepair
 // (potential) a point inside the cut-offs lies above them: 1 + T can be small or
 // negative there, and a fast pass renormalises after every point
 #define EPSCU_STATUS_STEEP 0x40000
-// (potential) ... so far above that 1 + T is negative there at some energy of the
-// range: the sign changes of a lane pass's state, u times the product of the f
-// before it, are then not the levels below E wherever u changes sign at such a
-// point or does not (0.1% of the energies, next to levels of the well on that
-// side, up to 2 off); the scans count those potentials point by point
+// (potential) ... so far above that f = 1 + T is negative there at some energy of
+// the range.  A lane pass counts the sign changes of u times the product of the
+// f before it, which are the levels below E only while u changes sign at every
+// such point (all but ~0.1% of the energies, those next to the levels of the
+// well on one side: up to 2 off), so the scans count these potentials point by
+// point and their close levels take the group passes
 #define EPSCU_STATUS_BELOW 0x100000
 #define EPSCU_STATUS_PUBLIC 0xffff
 // spacing of the samples of the twist-index search
