@@ -46,7 +46,7 @@ struct Side64 {
 };
 
 // STEEP: f may be anything (a barrier above the cut-offs); otherwise f >= 1/2, and
-// its reciprocal needs no look at its range (4% of a solve of 2900 x 20 points)
+// its reciprocal needs no look at its range (4% of a small batch, 5.84 -> 6.07 ms)
 template <bool WRITE, bool STEEP>
 __device__ __forceinline__ void side64_of(const double* __restrict__ W, double aE, int from, int to, int dir, Side64& st,
                                           double* __restrict__ out, double L, int Xk) {
